@@ -20,12 +20,13 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
 UNITS = {
     "implsch.cu": [],
+    "implsch_tile.cu": [],
     "propags.cu": ["-fmad=false"],
     "api.cu": [],
     "adjoint.cu": [],
     "output.cu": ["-fmad=false"],
 }
-HEADERS = ["implsch.cuh", "propags.cuh", "propargs.hpp", "devmath.cuh", "kernels.hpp", "adjoint.cuh", "adjoint_warp.cuh", "spectral_tables.hpp", "wamgpu_config.hpp"]
+HEADERS = ["implsch.cuh", "implsch_tile.cuh", "propags.cuh", "propargs.hpp", "devmath.cuh", "kernels.hpp", "adjoint.cuh", "adjoint_warp.cuh", "spectral_tables.hpp", "wamgpu_config.hpp"]
 
 
 def _nvcc():

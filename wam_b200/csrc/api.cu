@@ -55,9 +55,11 @@ struct wamgpu_ctx {
   cudaStream_t stream = nullptr;
   cudaStream_t copy_stream = nullptr;  // host->device copies overlapped with the kernels of a host-buffer step
   cudaStream_t down_stream = nullptr;  // device->host copies of a host-buffer step
+  cudaStream_t src_stream[4] = {};     // IMPLSCH of the chunks of a host-buffer step (made at its first call)
   std::vector<cudaEvent_t> xfer_ev;     // ordering events between the two streams
   int nsm = 148;
-  int P = 8;  // sea points per IMPLSCH CTA
+  int P = 8;  // sea points per IMPLSCH CTA of the warp-per-point kernel
+  int wave = 0;  // sea points that kernel holds on the chip at once
   // grid (reference convention, host)
   int nsea = 0, ny = 0, n_ext = 0;
   int halo = 0;  // largest |neighbour - point| over KLAT/KLON (sea point numbers)
@@ -146,6 +148,43 @@ template <typename T> cudaError_t upload(DevBuf& b, const std::vector<T>& h, cud
   if (e != cudaSuccess) return e;
   if (h.empty()) return cudaSuccess;
   return cudaMemcpyAsync(b.p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, s);
+}
+
+// Whether the DIA has the geometry that IMPLSCH on tiles is written for: the
+// partner tables K11W/K21W one direction beside K1W/K2W, outwards of the
+// centre in both KH, and the rows of an MC at MC+2, MC+3, MC-4, MC-3, clamped
+// to the spectrum where they are gathered.  Frequency ratio 1.1 and the
+// reference's quadruplet give both.
+template <typename R> bool tile_geometry(const TableSet<R>& t) {
+  const int KL = t.KL, ML = t.ML;
+  auto off = [&](const std::vector<int>& tb, int kh) { return tb[KL * kh] - 1; };
+  auto turn = [&](int o, int by) { return (o + by + KL) % KL; };
+  if (off(t.K11W, 0) != turn(off(t.K1W, 0), -1) || off(t.K11W, 1) != turn(off(t.K1W, 1), 1) ||
+      off(t.K21W, 0) != turn(off(t.K2W, 0), 1) || off(t.K21W, 1) != turn(off(t.K2W, 1), -1) || t.MLSTHG != ML + 4)
+    return false;
+  for (int mc = 1; mc <= t.MLSTHG; ++mc) {
+    const int i = mc - t.MFRSTLW;
+    const int* ii = &t.INLCOEF[5 * (mc - 1)];
+    auto in = [&](int m) { return std::min(std::max(m, 1), ML); };
+    if (ii[0] != in(mc) || ii[1] != in(mc + 2) || ii[2] != in(mc + 3) || ii[3] != in(mc - 4) || ii[4] != in(mc - 3))
+      return false;
+    // target rows: outside the spectrum they are clamped or skipped
+    if (t.IKP[i] != mc + 2 || t.IKP1[i] != mc + 3 || (mc > 4 && t.IKM[i] != mc - 4) || (mc > 3 && t.IKM1[i] != mc - 3))
+      return false;
+  }
+  return true;
+}
+
+// Sea points per IMPLSCH CTA: 32 where the context runs on tiles, else those
+// of the warp-per-point kernel.  Tiles from the first point that the warps no
+// longer hold at once: up to there that kernel takes one wave, and a point of
+// its own per warp is done sooner than a tile (135 points, ST4, KL=24: 151 us
+// against 182; 1485 points, ST6, KL=36: 84 against 121), beyond it takes two and
+// more (1800 points: 302 against 182, 149 against 120).  The rule looks at the
+// context's whole grid, so chunks, owned ranges and ensemble members of one
+// context all run on the same kernel and agree bit for bit.
+template <typename R> int cta_points(const wamgpu_ctx* ctx, const DevTables<R>& d) {
+  return d.tile.smem && ctx->nsea > ctx->wave ? 32 : ctx->P;
 }
 
 template <typename R> int build_tables(wamgpu_ctx* ctx, Impl<R>& I) {
@@ -393,8 +432,14 @@ template <typename R> int build_tables(wamgpu_ctx* ctx, Impl<R>& I) {
     int ctas = std::min(32 / P, (int)(smpersm / (need + 1024)));
     if (P * ctas > best_warps) { best_warps = P * ctas; ctx->P = P; }
   }
+  ctx->wave = best_warps * ctx->nsm;
   if (ctx->P) CK(implsch_set_max_smem<R>(ctx->P, implsch_smem_bytes(d, ctx->P)), "smem attribute");
   if (!ctx->P) return fail(ctx, WAMGPU_E_ARG, "spectrum too large for the shared-memory workspace");
+  if constexpr (sizeof(R) == 4) {
+    // 1 KB is left to the batched kernel's static part
+    if (tile_geometry(t)) d.tile = tile_shape(d, maxsm - 1024);
+    if (d.tile.smem) CK(tile_set_max_smem(d), "smem attribute");
+  }
   CK(cudaStreamSynchronize(s), "table upload");
   return WAMGPU_OK;
 }
@@ -636,7 +681,7 @@ int implsch_dev_t(wamgpu_ctx* ctx, Impl<R>& I, void* fl3, int ld, const void* u1
     a.diag_ll = ctx->diag_ll ? ctx->diag_ll + p0 : nullptr;
     a.diag_ld = ctx->diag_ld;
   }
-  { TimedLaunch tl(ctx, 1, s); CK(launch_implsch<R>(I.dt, a, ctx->P, s), "implsch launch"); }
+  { TimedLaunch tl(ctx, 1, s); CK(launch_implsch<R>(I.dt, a, cta_points(ctx, I.dt), s), "implsch launch"); }
   return WAMGPU_OK;
 }
 
@@ -1357,7 +1402,11 @@ int step_host_t(wamgpu_ctx* ctx, Impl<R>& I, float* fl3, int nprop, const float*
   // precedes sub-step j+1 of chunk q-1, which overwrites its input; and
   // IMPLSCH of chunk q follows the last sub-step of chunks q-1..q+1.
   const int width = std::max(ctx->halo, 1);
-  const int nq = n > 0 ? std::min(64, std::max(1, n / width)) : 1;
+  // At most 64 chunks, and none below 1184 points (37 tiles of IMPLSCH, a
+  // quarter of the SMs for each of the four in flight) beyond the fourth:
+  // below that the launches bound the step (30k points: 64 chunks 8.2 ms, 32
+  // and 16 chunks 4.7 ms; 756k points: 64 chunks 82 ms, 32 chunks 90 ms).
+  const int nq = n > 0 ? std::min({64, std::max(1, n / width), std::max(4, n / 1184)}) : 1;
   std::vector<int> lo(nq + 1);
   {
     // The first nsub+2 chunks are small (a quarter of the others, and at least
@@ -1377,7 +1426,7 @@ int step_host_t(wamgpu_ctx* ctx, Impl<R>& I, float* fl3, int nprop, const float*
   // copies move pieces of kChunksPerCopy chunks
   const int cpc = kChunksPerCopy, npc = (nq + cpc - 1) / cpc;
   auto piece_lo = [&](int p) { return lo[std::min(nq, p * cpc)]; };
-  const int nev = 2 * npc;
+  const int nev = 2 * npc + nq;  // uploads, downloads, last sub-steps
   if ((int)ctx->xfer_ev.size() < nev)
     for (int i = (int)ctx->xfer_ev.size(); i < nev; ++i) {
       cudaEvent_t e;
@@ -1385,6 +1434,8 @@ int step_host_t(wamgpu_ctx* ctx, Impl<R>& I, float* fl3, int nprop, const float*
       ctx->xfer_ev.push_back(e);
     }
   cudaStream_t d = ctx->down_stream;
+  for (cudaStream_t& x : ctx->src_stream)
+    if (!x) CK(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking), "stream");
   // the spectrum piece by piece (the per-point fields went up on s above)
   for (int p = 0; p < npc; ++p) {
     const int a0 = piece_lo(p);
@@ -1413,6 +1464,12 @@ int step_host_t(wamgpu_ctx* ctx, Impl<R>& I, float* fl3, int nprop, const float*
     if (q < 0 || q >= nq) continue;
     if (nsub == 0) { int rc = ready(q); if (rc) return rc; }
     const int p0 = lo[q], p1 = lo[q + 1];
+    // IMPLSCH of consecutive chunks on four streams in turn: a chunk is a few
+    // tiles, far fewer than the SMs, and no later sub-step reads or writes the
+    // chunk (those of key t + 1 and on start at chunk q + 2)
+    cudaStream_t si = ctx->src_stream[q & 3];
+    CK(cudaEventRecord(ctx->xfer_ev[2 * npc + q], s), "event");
+    CK(cudaStreamWaitEvent(si, ctx->xfer_ev[2 * npc + q], 0), "wait");
     if (p1 > p0) {
       ImplArgs<R> a;
       a.nsea = p1 - p0; a.ld = n;
@@ -1426,11 +1483,11 @@ int step_host_t(wamgpu_ctx* ctx, Impl<R>& I, float* fl3, int nprop, const float*
       a.status = I.status.template as<int>();
       a.enh = I.has_enh ? I.enh.template as<R>() + p0 : nullptr; a.enh_ld = n;
       a.wncg = ctx->wncg_valid ? I.wncg.template as<R>() + (size_t)p0 * 2 * ctx->cfg.ml : nullptr;
-      { TimedLaunch tl(ctx, 1, s); CK(launch_implsch<R>(I.dt, a, ctx->P, s), "implsch launch"); }
+      { TimedLaunch tl(ctx, 1, si); CK(launch_implsch<R>(I.dt, a, cta_points(ctx, I.dt), si), "implsch launch"); }
     }
     if (q % cpc == cpc - 1 || q == nq - 1) {  // the last chunk of a piece: the piece goes down
       const int pc = q / cpc, a0 = piece_lo(pc);
-      CK(cudaEventRecord(ctx->xfer_ev[npc + pc], s), "event");
+      CK(cudaEventRecord(ctx->xfer_ev[npc + pc], si), "event");
       CK(cudaStreamWaitEvent(d, ctx->xfer_ev[npc + pc], 0), "wait");
       const size_t w = (size_t)(piece_lo(pc + 1) - a0) * 4;
       if (w) CK(cudaMemcpy2DAsync(fl3 + a0, (size_t)n * 4, f3 + a0, (size_t)n * 4, w, (size_t)KL * ML,
@@ -1443,6 +1500,7 @@ int step_host_t(wamgpu_ctx* ctx, Impl<R>& I, float* fl3, int nprop, const float*
   CK(cudaMemcpyAsync(z0, I.z0.template as<R>(), (size_t)n * 4, cudaMemcpyDeviceToHost, d), "D2H");
   CK(cudaStreamSynchronize(d), "step copies");
   CK(cudaStreamSynchronize(c), "step copies");
+  for (cudaStream_t x : ctx->src_stream) CK(cudaStreamSynchronize(x), "step sync");
   CK(cudaStreamSynchronize(s), "step sync");
   return wamgpu_sync(ctx);
 }
@@ -1563,6 +1621,13 @@ std::vector<double> source_key(const Config& c) {
           double(c.ndepth), c.deptha, c.depthd, double(c.precision)};
 }
 
+// Members of one launch also run on the same kernel (cta_points).
+template <typename R> std::vector<double> member_key(wamgpu_ctx* c) {
+  std::vector<double> k = source_key(c->cfg);
+  k.push_back(cta_points(c, impl_of<R>(c).dt) == 32);
+  return k;
+}
+
 // IMPLSCH member lists, one per source-table class, largest members first
 // (their CTAs start first).  For tuning (out != null) each member reads its
 // current spectrum and writes `out`, TAUW/USTAR/Z0 go to `tmp3` and the
@@ -1574,7 +1639,7 @@ int batch_impl_lists(wamgpu_batch* b, const std::vector<int>& Pin, std::vector<B
   std::vector<std::vector<double>> keys;
   std::vector<int> cls(n);
   for (int g = 0; g < n; ++g) {
-    std::vector<double> k = source_key(b->members[g]->cfg);
+    std::vector<double> k = member_key<R>(b->members[g]);
     auto it = std::find(keys.begin(), keys.end(), k);
     cls[g] = (int)(it - keys.begin());
     if (it == keys.end()) keys.push_back(k);
@@ -1586,8 +1651,10 @@ int batch_impl_lists(wamgpu_batch* b, const std::vector<int>& Pin, std::vector<B
     for (int g = 0; g < n; ++g) if (cls[g] == (int)ci) order.push_back(g);
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return b->members[x]->nsea > b->members[y]->nsea; });
     // sea points per CTA: the tuned value of this class, else the contexts' own occupancy choice
-    const int P = (ci < Pin.size() && Pin[ci] > 0) ? Pin[ci] : b->members[order[0]]->P;
-    if (implsch_smem_bytes(impl_of<R>(b->members[order[0]]).dt, P) + sizeof(ImplArgs<R>) + 64 > kMaxSmemPerCta)
+    const DevTables<R>& dt = impl_of<R>(b->members[order[0]]).dt;
+    const bool tile = cta_points(b->members[order[0]], dt) == 32;
+    const int P = tile ? 32 : (ci < Pin.size() && Pin[ci] > 0) ? Pin[ci] : b->members[order[0]]->P;
+    if (!tile && implsch_smem_bytes(dt, P) + sizeof(ImplArgs<R>) + 64 > kMaxSmemPerCta)
       return bfail(b, WAMGPU_E_ARG, "points per CTA too large for a member");
     std::vector<ImplArgs<R>> mem(order.size());
     std::vector<int> first(order.size() + 1, 0);
@@ -1617,8 +1684,11 @@ int batch_impl_lists(wamgpu_batch* b, const std::vector<int>& Pin, std::vector<B
     BatchList& L = Ls[ci];
     L.family = order[0];  // whose source tables the launch passes
     L.P = P;
-    L.smem = implsch_smem_bytes(impl_of<R>(b->members[order[0]]).dt, P);
-    BCK(implsch_set_max_smem<R>(P, L.smem), "smem attribute");
+    L.smem = 0;
+    if (!tile) {
+      L.smem = implsch_smem_bytes(dt, P);
+      BCK(implsch_set_max_smem<R>(P, L.smem), "smem attribute");
+    }
     BCK(upload_vec(L.mem, mem, s), "upload batch");
     BCK(upload_vec(L.first, first, s), "upload batch");
     L.nmem = (int)order.size(); L.nblocks = first.back();
@@ -1772,8 +1842,9 @@ template <typename R> int batch_tune(wamgpu_batch* b, cudaStream_t s, int* P_out
   for (int P : cands) {
     if (rc) break;
     std::vector<int> Pin(ncls, P);
-    for (size_t ci = 0; ci < ncls; ++ci)  // classes this shape does not fit keep their default
-      if (implsch_smem_bytes(impl_of<R>(b->members[b->imp[ci].family]).dt, P) + sizeof(ImplArgs<R>) + 64 > kMaxSmemPerCta)
+    for (size_t ci = 0; ci < ncls; ++ci)  // classes on tiles, and those this shape does not fit, keep their default
+      if (b->imp[ci].P == 32 ||
+          implsch_smem_bytes(impl_of<R>(b->members[b->imp[ci].family]).dt, P) + sizeof(ImplArgs<R>) + 64 > kMaxSmemPerCta)
         Pin[ci] = 0;
     std::vector<BatchList> Ls;
     if ((rc = batch_impl_lists<R>(b, Pin, Ls, &out, &t3, tstatus.template as<int>(), s))) break;
@@ -1796,12 +1867,16 @@ template <typename R> int batch_tune(wamgpu_batch* b, cudaStream_t s, int* P_out
   b->built = false;
   if ((rc = batch_build<R>(b, s))) return rc;
   if (P_out) {  // the shape of the class with the most sea points
-    size_t best = 0; int pc = b->imp.empty() ? 0 : b->imp[0].P;
+    // (classes on tiles have no such shape: their context's own choice)
+    auto shape = [&](size_t ci) {
+      return b->imp[ci].P == 32 ? b->members[b->imp[ci].family]->P : b->imp[ci].P;
+    };
+    size_t best = 0; int pc = b->imp.empty() ? 0 : shape(0);
     for (size_t ci = 0; ci < b->imp.size(); ++ci) {
       size_t pts = 0;
       for (size_t g = 0; g < b->members.size(); ++g)
-        if (source_key(b->members[g]->cfg) == source_key(b->members[b->imp[ci].family]->cfg)) pts += b->members[g]->nsea;
-      if (pts > best) { best = pts; pc = b->imp[ci].P; }
+        if (member_key<R>(b->members[g]) == member_key<R>(b->members[b->imp[ci].family])) pts += b->members[g]->nsea;
+      if (pts > best) { best = pts; pc = shape(ci); }
     }
     *P_out = pc;
   }
@@ -1854,12 +1929,14 @@ int wamgpu_destroy(wamgpu_ctx* ctx) {
   if (ctx->stream) { cudaSetDevice(ctx->cfg.device); cudaStreamSynchronize(ctx->stream); }
   if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
   if (ctx->down_stream) cudaStreamSynchronize(ctx->down_stream);
+  for (cudaStream_t x : ctx->src_stream) if (x) cudaStreamSynchronize(x);
   ctx->impl.reset();
   for (int c = 0; c < 2; ++c) for (auto& e : ctx->ev[c]) ctx->ev_pool.push_back(e);
   for (auto& e : ctx->ev_pool) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
   for (auto e : ctx->xfer_ev) cudaEventDestroy(e);
   if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
   if (ctx->down_stream) cudaStreamDestroy(ctx->down_stream);
+  for (cudaStream_t x : ctx->src_stream) if (x) cudaStreamDestroy(x);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return WAMGPU_OK;

@@ -47,6 +47,33 @@ __device__ __forceinline__ float radd(float a, float b) { return __fadd_rn(a, b)
 __device__ __forceinline__ double radd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ float rsub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ double rsub(double a, double b) { return __dsub_rn(a, b); }
+// Two single-precision operations per instruction (fma.rn.f32x2 and the like):
+// each half rounds as the scalar operation does, but the compiler fuses an add2
+// of a mul2 into one rounding, .rn or not (seen on sm_100a, CUDA 12.9): sums of
+// products that must round twice stay scalar.  A packed operation issues in one
+// slot and takes the FP32 pipe two cycles (B200): it saves issue slots only.
+struct F2 {
+  unsigned long long v;
+  __device__ F2() {}
+  __device__ F2(float x, float y) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(x), "f"(y)); }
+  __device__ float x() const { float a, b; asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); return a; }
+  __device__ float y() const { float a, b; asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); return b; }
+};
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return d;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+  F2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+  return d;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+  return d;
+}
 // Quotients a / b for one divisor b, each rounded as the IEEE division
 // rounds it, without a division per quotient.  In single precision the
 // quotient is the float rounding of a times the double reciprocal of b.  That
@@ -60,12 +87,41 @@ template <> struct RecipDiv<float> {
   double y;
   __device__ explicit RecipDiv(float b) : y(1.0 / (double)b) {}
   __device__ float operator()(float a) const { return __double2float_rn(__dmul_rn((double)a, y)); }
+  __device__ F2 operator()(F2 a) const { return F2((*this)(a.x()), (*this)(a.y())); }
 };
 template <> struct RecipDiv<double> {
   double b;
   __device__ explicit RecipDiv(double b_) : b(b_) {}
   __device__ double operator()(double a) const { return a / b; }
 };
+// The same quotients without leaving single precision: with y the correctly
+// rounded reciprocal of b, two corrections by the exact residual a - q*b end in
+// the correctly rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990), as
+// long as the residual is exact, which holds for a = 0 and for |a| >= LO
+// (b and the quotient in the normal range).  The caller checks that and takes
+// RecipDiv otherwise.  Why: the conversions to and from double run at 1/8 of
+// the FP32 rate; a RecipDiv quotient takes 4.2 cycles per warp and SM, this 1.4
+// (B200).
+struct MarksteinDiv {
+  static constexpr float LO = 1e-28f;  // 2^-100 and room for a divisor of a hundred in between
+  float b, y;
+  __device__ explicit MarksteinDiv(float b_) : b(b_), y(1.0f / b_) {}
+  __device__ float operator()(float a) const {
+    float q = __fmul_rn(a, y);
+    q = __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+    return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+  }
+  __device__ F2 operator()(F2 a) const {
+    const F2 y2(y, y), nb(-b, -b);
+    F2 q = mul2(a, y2);
+    q = fma2(fma2(q, nb, a), y2, q);
+    return fma2(fma2(q, nb, a), y2, q);
+  }
+};
+// Running test of the numerators: bits - 1 of |a| as an unsigned number is
+// smallest for the smallest nonzero |a| (zero wraps to the largest).
+__device__ __forceinline__ unsigned num_bits(float a) { return (__float_as_uint(a) & 0x7fffffffu) - 1u; }
+
 // Correctly rounded single-precision transcendentals (evaluated in double,
 // rounded once) for the same per-point values: the cut-off index's LOG10 /
 // LOG, the LFACTOR exponentials and wind-direction cosines, and WAVNU2's

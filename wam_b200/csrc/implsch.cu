@@ -193,6 +193,8 @@ template <typename R> cudaError_t implsch_set_max_smem(int P, size_t bytes) {
 
 template <typename R> cudaError_t launch_implsch(const DevTables<R>& T, const ImplArgs<R>& a, int P, cudaStream_t s) {
   if (a.nsea == 0) return cudaSuccess;
+  if constexpr (sizeof(R) == 4)
+    if (P == 32) return launch_implsch_tile(T, a, s);
   size_t smem = implsch_smem_bytes(T, P);
   if (sizeof(R) == 4) {
     if (P == 4) launch_one<R, 4>(T, a, smem, s);
@@ -211,6 +213,8 @@ template <typename R>
 cudaError_t launch_implsch_batch(const DevTables<R>& T, const ImplArgs<R>* mem, const int* first, int nmem, int nblocks,
                                  int P, size_t smem, cudaStream_t s) {
   if (nblocks == 0) return cudaSuccess;
+  if constexpr (sizeof(R) == 4)
+    if (P == 32) return launch_implsch_tile_batch(T, mem, first, nmem, nblocks, s);
   if (sizeof(R) == 4) {
     if (P == 4) launch_batch_one<R, 4>(T, mem, first, nmem, nblocks, smem, s);
     else if (P == 6) launch_batch_one<R, 6>(T, mem, first, nmem, nblocks, smem, s);

@@ -37,6 +37,7 @@ template <typename R> struct ImplArgs {
   R* lfout = nullptr;  // ST6: per point the RTAU of LFACTOR's last round (0 without one), or null
 };
 
+// points_per_cta: 32 for tiles (single precision, T.tile.smem != 0), else a shape of the warp-per-point kernel.
 template <typename R> cudaError_t launch_implsch(const DevTables<R>& T, const ImplArgs<R>& a, int points_per_cta, cudaStream_t s);
 // WAVNU2's wavenumber and group velocity of every (sea point, frequency) from
 // the depth, the same routine the ST6 step uses: out[ij * 2*ML + m] = WN,
@@ -49,6 +50,13 @@ template <typename R> cudaError_t launch_wavnu2(const DevTables<R>& T, const R* 
 template <typename R>
 cudaError_t launch_implsch_batch(const DevTables<R>& T, const ImplArgs<R>* mem, const int* first, int nmem, int nblocks,
                                  int points_per_cta, size_t smem, cudaStream_t s);
+// IMPLSCH on tiles of 32 sea points, single precision (T.tile.smem != 0): one
+// context, and the batched form (first[] counts CTAs of 32 points).
+TileShape tile_shape(const DevTables<float>& T, int max_smem);
+cudaError_t tile_set_max_smem(const DevTables<float>& T);
+cudaError_t launch_implsch_tile(const DevTables<float>& T, const ImplArgs<float>& a, cudaStream_t s);
+cudaError_t launch_implsch_tile_batch(const DevTables<float>& T, const ImplArgs<float>* mem, const int* first, int nmem,
+                                      int nblocks, cudaStream_t s);
 template <typename R> size_t implsch_smem_bytes(const DevTables<R>& T, int points_per_cta);
 template <typename R> cudaError_t implsch_set_max_smem(int points_per_cta, size_t bytes);
 

@@ -37,6 +37,15 @@ struct SmallLayout {
   int nint;
 };
 
+// Shape and shared-memory layout of IMPLSCH on tiles of 32 sea points
+// (implsch_tile.cuh); smem = 0 where it does not apply.
+struct TileShape {
+  int dpw, nw;                // directions per warp, warps
+  int nbuf, xcol;             // DIA exchange buffers and their columns (KL + dpw wrapped copies)
+  int oTab, oU, oRow, oLL;    // word offsets: tables, union region, per-frequency rows, wind-sea mask
+  int smem;                   // bytes
+};
+
 // Everything the kernels need besides the per-point fields; passed by value.
 template <typename R> struct DevTables {
   int KL, ML, NS, NDEPTH, MFRSTLW, MLSTHG, KFRH, NSDSNTH, NK10;
@@ -46,6 +55,7 @@ template <typename R> struct DevTables {
   int iphys, shallow, isnonlin, lcflx;
   R DELTH, DELTR, INV_LOG_CO, MO_TAIL, MM1_TAIL, DELU, DAL1, DAL2, X0TAUHF;
   R BETAMAX, ZALP, ALPHA, TAUWSHELTER, CDFAC, DELT;
+  TileShape tile;
   SmallLayout lay;
   const R* small;      // packed float tables (global copy)
   const int* ismall;   // packed int tables (global copy)
