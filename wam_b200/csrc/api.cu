@@ -563,6 +563,15 @@ template <typename R> int prepare_prop(wamgpu_ctx* ctx, Impl<R>& I, float* total
   A.TCGOND = I.tcgond.template as<R>(); A.TSIHKD = I.tsihkd.template as<R>(); A.TFAK = I.tfak.template as<R>();
   A.GOM = I.gom.template as<R>(); A.FR = I.fr.template as<R>();
   for (int k = 0; k < KL; ++k) { A.sinth[k] = t.SINTH[k]; A.costh[k] = t.COSTH[k]; }
+  {
+    int ns = 0;
+    for (int k = 1; k <= KL; ++k)
+      if (k == KL || (A.sinth[k] >= R(0.)) != (A.sinth[k - 1] >= R(0.)) || (A.costh[k] >= R(0.)) != (A.costh[k - 1] >= R(0.))) {
+        if (ns < 8) A.seg[ns] = k;
+        ++ns;
+      }
+    if (ns > 8) A.seg[0] = 0;
+  }
   // CHECK_CFL (:1917-2138) from the extrema of the recomputed coefficients
   CK(I.cflext.ensure(2 * CFL_NCLASS * sizeof(long long)), "alloc");
   CK(launch_cfl_extrema<R>(A, I.cflext.template as<long long>(), ctx->nsm, s), "cfl kernel");
@@ -1738,8 +1747,9 @@ template <typename R> int batch_build(wamgpu_batch* b, cudaStream_t s) {
         M.dst = (it % 2 == 0) ? sc : f3;
         M.ld = b->st[g].ld;
         M.nbi = (A.i1 - A.i0 + b->bs - 1) / b->bs;
+        M.pair = propags_pairs(A, M.ld);
         mem.push_back(M);
-        first.push_back(first.back() + c->cfg.ml * M.nbi);
+        first.push_back(first.back() + (M.pair ? (c->cfg.ml + 1) / 2 : c->cfg.ml) * M.nbi);
       }
       BatchList& L = b->sub[it][f];
       L.family = rep;

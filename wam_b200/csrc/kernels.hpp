@@ -73,11 +73,18 @@ template <typename R> struct PropMember {
   const R* src;
   R* dst;
   int ld, nbi;
+  int pair;  // two frequencies per CTA (propags_pairs)
 };
+// Whether a sub-step takes two frequencies per thread: variants without
+// currents, 32-bit offsets in a plane, at most eight segments of directions.
+bool propags_planes_independent(int variant);
+template <typename R> bool propags_pairs(const PropArgs<R>& A, int ld) {
+  return propags_planes_independent(A.variant) && A.seg[0] > 0 && (size_t)ld * A.KL < (size_t(1) << 31);
+}
 // All members of one coefficient family (variant, reduced grid, depth
 // refraction taken from `family`) in one launch of bs-point CTAs (128 or 256);
 // CTA b works for member g with first[g] <= b < first[g+1] (first[g] = sum of
-// ML*nbi over the members before g).
+// ML*nbi, or (ML+1)/2*nbi with pairs, over the members before g).
 template <typename R>
 cudaError_t launch_propags_batch(const PropArgs<R>& family, const PropMember<R>* mem, const int* first, int nmem,
                                  int nblocks, int bs, cudaStream_t s);

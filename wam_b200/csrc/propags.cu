@@ -50,69 +50,250 @@ __global__ void __launch_bounds__(128) propags_kernel(const __grid_constant__ Pr
   propags_point<R, VAR, RED, REFRD>(A, f1, ld1, f3, ld3, i, m0 + blockIdx.y);
 }
 
-// Two frequencies m, m+1 of one sea point per thread, for the variants
-// without currents (a sub-step of plane m then reads plane m only).  The
-// direction-dependent work that does not depend on the frequency (direction
-// tables, upwind neighbour choice and addresses, |SIN|, |COS| and the metric
-// products, the depth-gradient part of THDD) is the same expression for both
-// frequencies and is formed once; every coefficient still gets the
-// reference's operations, so the result equals the one-frequency kernel's.
-// With mb beyond the planes (odd count) the second frequency repeats the
-// first and is not stored.
-template <typename R, int VAR, bool RED, bool REFRD>
-__device__ __forceinline__ void propags_point2(const PropArgs<R>& A, const R* __restrict__ f1, int ld1,
-                                               R* __restrict__ f3, int ld3, int i, int m, bool two) {
+// The stencil for the variants without currents, two frequencies m, m+1 of one
+// sea point per thread (a sub-step of plane m reads plane m only).  Issue-bound
+// work, so what the coefficients of Site::coef_w recompute is formed once, with
+// the same operations and hence the same bits:
+//   - the boundary term of directions k and k+1 (DTP of k) is also DTM of k+1:
+//     its sums and products commute, so one value per direction serves both,
+//     and its share of direction k+1 is multiplied by F(k) at once;
+//   - products that depend on the point and the frequency alone (group velocity
+//     sums of the neighbours, DRGM*CG) are formed before the loop;
+//   - which neighbour is upwind changes with the signs of SIN and COS only: the
+//     directions go in segments of constant signs (A.seg), the selection is made
+//     per segment, and the loop inside has no branch, so that it unrolls with
+//     the loads of three directions in flight;
+//   - a land neighbour is read as the point itself and replaced by 0;
+//   - row offsets are 32-bit and run along;
+//   - CHECK_CFL's division by COUNTER runs as an exact scaled Markstein quotient.
+// 105 -> 67 thread instructions per bin (32 of them FP32) on the shallow
+// spherical grid with depth refraction.  A sub-step of 756k points, 36x30, takes
+// 1.98 ms (3.3 TB/s of algorithmic traffic) against 2.69 before, with COUNTER = 2
+// on 159k points 36x35 0.67 against 1.39, deep on 47k points 24x25 0.074 against
+// 0.100.  Now bound by issue (71 % of the slots) and the latency of L2: three
+// directions in flight are the most that 64 registers hold (unrolled by 1, 2 or
+// 4 without the prefetch below: 4.1, 3.5 and 2.8 ms); the leaner deep stencil
+// takes six.
+// x / COUNTER, rounded as the division rounds it.
+template <typename R> struct CounterDiv;
+template <> struct CounterDiv<float> {
+  float b, y;
+  __device__ explicit CounterDiv(float rc) : b(rc), y(1.0f / rc) {}
+  // scaled by 2^60, the residuals are exact for every coefficient (at most
+  // COUNTER in size), and so is the way back above 2^-126
+  __device__ float operator()(float x) const {
+    const float a = x * 1152921504606846976.f;
+    float q = a * y;
+    q = __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+    q = __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+    return q * 8.67361737988403547e-19f;
+  }
+};
+template <> struct CounterDiv<double> {
+  double b;
+  __device__ explicit CounterDiv(double rc) : b(rc) {}
+  __device__ double operator()(double x) const { return x / b; }
+};
+
+// What one frequency of a point carries along the directions.
+template <typename R> struct Line {
+  R kS, kN, kW, kE;      // factors of the south, north, west and east boundary
+  R drc, tsi;            // DRGM*CG, depth refraction factor
+  R fk;                  // F(k)
+  R mn;                  // negative part of DTM
+  R up;                  // positive part of DTM (over COUNTER) times F(k-1)
+  R th;                  // THDD(k)
+};
+
+template <typename R, int VAR, bool RED, bool REFRD, bool CNT>
+__device__ __forceinline__ void propags_pair(const PropArgs<R>& A, const R* __restrict__ f1, int ld1, R* __restrict__ f3,
+                                             int ld3, int i, int m, bool two) {
   using S = Site<R, VAR, RED, REFRD>;
-  static_assert(!S::CUR, "two-frequency PROPAGS is for the variants without currents");
-  const int mb = two ? m + 1 : m;
-  const S sa(A, i, m), sb(A, i, mb);
-  const int KL = A.KL;
-  const size_t plane = (size_t)ld1 * KL;
-  const R* fa = f1 + plane * m;
-  const R* fb = f1 + plane * mb;
-  const bool theta = REFRD || S::SPH;
-  auto at = [&](const R* fm, int p1, int k) -> R { return p1 == 0 ? R(0) : __ldg(&fm[(p1 - 1) + (size_t)ld1 * k]); };
-  R fkm_a = at(fa, i + 1, KL - 1), fk_a = at(fa, i + 1, 0);
-  R fkm_b = at(fb, i + 1, KL - 1), fk_b = at(fb, i + 1, 0);
-  R* outa = f3 + i + (size_t)ld3 * KL * m;
-  R* outb = f3 + i + (size_t)ld3 * KL * mb;
-  typename S::Win Wa = sa.window(0), Wb = sb.window(0);
-  for (int k = 0; k < KL; ++k) {
-    const int kp = (k + 1 == KL) ? 0 : k + 1;
-    const R fkp_a = at(fa, i + 1, kp), fkp_b = at(fb, i + 1, kp);
-    const Coefs<R> ca = sa.coef_w(Wa), cb = sb.coef_w(Wb);
-    const bool ic0 = Wa.cs >= R(0.), is0 = Wa.sn >= R(0.);
-    const int pl = ic0 ? sa.s0 : sa.n0, pw = is0 ? sa.w0 : sa.e0;
-    R va = ca.sum * fk_a + ca.lat11 * at(fa, pl, k) + ca.lon1 * at(fa, pw, k);
-    R vb = cb.sum * fk_b + cb.lat11 * at(fb, pl, k) + cb.lon1 * at(fb, pw, k);
-    if (theta) { va = va + ca.th1 * fkp_a + ca.th2 * fkm_a; vb = vb + cb.th1 * fkp_b + cb.th2 * fkm_b; }
-    if (RED) {
-      const int p2 = ic0 ? sa.s1 : sa.n1;
-      va = va + ca.lat12 * at(fa, p2, k);
-      vb = vb + cb.lat12 * at(fb, p2, k);
+  static_assert(!S::CUR, "the pair stencil is for the variants without currents");
+  constexpr bool SH = S::SH, SPH = S::SPH, THETA = SPH || (SH && REFRD), TH = SH && REFRD;
+  constexpr int UN = SH || CNT ? 3 : 6;  // directions whose loads are in flight
+  const int KL = A.KL, mb = two ? m + 1 : m;
+  const R one = R(1.), z = R(0.);
+  unsigned iS, iN, iW, iE, iS2 = 0, iN2 = 0;  // neighbours' indices, the point's own for land
+  bool lS, lN, lW, lE, lS2 = false, lN2 = false;
+  R wl1 = one, wl2 = one, d0, ddphi = z, ddlam = z, gom[2] = {z, z};
+  Line<R> L[2];
+  {
+    auto nb = [&](int p1, unsigned& idx, bool& land) { land = p1 == 0; idx = land ? (unsigned)i : (unsigned)(p1 - 1); };
+    const S sa(A, i, m), sb(A, i, mb);
+    nb(sa.s0, iS, lS); nb(sa.n0, iN, lN); nb(sa.w0, iW, lW); nb(sa.e0, iE, lE);
+    if (RED) { nb(sa.s1, iS2, lS2); nb(sa.n1, iN2, lN2); wl1 = sa.wl1; wl2 = sa.wl2; }
+    d0 = sa.d0;
+    if (TH) { ddphi = sa.ddphi; ddlam = sa.ddlam; }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const S& s = q ? sb : sa;
+      Line<R>& l = L[q];
+      gom[q] = s.gom;
+      if (SH) {
+        if (SPH && RED) {
+          l.kS = s.cg + s.ps * (s.wl1 * s.cgS + (one - s.wl1) * s.cgS1);
+          l.kN = s.cg + s.pn * (s.wl2 * s.cgN + (one - s.wl2) * s.cgN1);
+        } else if (SPH) { l.kS = s.cg + s.ps * s.cgS; l.kN = s.cg + s.pn * s.cgN; }
+        else { l.kS = s.cgS + s.cg; l.kN = s.cgN + s.cg; }
+        l.kW = s.cgW + s.cg; l.kE = s.cgE + s.cg;
+        l.drc = s.dr * s.cg; l.tsi = TH ? s.tsi : z;
+      } else {
+        l.kS = s.ps + one; l.kN = s.pn + one; l.kW = l.kE = one;
+        l.drc = s.dr; l.tsi = z;
+      }
     }
-    outa[(size_t)ld3 * k] = va;
-    if (two) outb[(size_t)ld3 * k] = vb;
-    fkm_a = fk_a; fk_a = fkp_a; fkm_b = fk_b; fk_b = fkp_b;
-    sa.advance(Wa, k);
-    sb.advance(Wb, k);
+  }
+  const CounterDiv<R> cd(CNT ? A.rcounter : one);
+  const R* fp[2] = {f1 + (size_t)ld1 * KL * m, f1 + (size_t)ld1 * KL * mb};
+  R* op[2] = {f3 + (size_t)ld3 * KL * m, f3 + (size_t)ld3 * KL * mb};
+  const unsigned ui = (unsigned)i, st1 = (unsigned)ld1, st3 = (unsigned)ld3;
+  // direction KL-1 to 0: the first DTM, F(KL-1), F(0)
+  const R snl = A.sinth[KL - 1], csl = A.costh[KL - 1];
+  R sn = A.sinth[0], cs = A.costh[0];
+  const R sp0 = A.DELTH0 * (sn + snl);
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    Line<R>& l = L[q];
+    const R fl = __ldg(fp[q] + st1 * (unsigned)(KL - 1) + ui);
+    l.fk = __ldg(fp[q] + ui);
+    R d = z;
+    l.th = z;
+    if (TH) {
+      l.th = (sn * ddphi - cs * ddlam) * l.tsi;
+      const R thm = (snl * ddphi - csl * ddlam) * l.tsi;
+      d = SPH ? l.drc * sp0 + (l.th + thm) * A.DELTHR : (l.th + thm) * A.DELTHR;
+    } else if (THETA) d = l.drc * sp0;
+    l.mn = dmin(z, d);
+    R th2 = dmax(z, d);
+    if (SPH && !SH) th2 = gom[q] * th2;
+    if (CNT) th2 = cd(th2);
+    l.up = th2 * fl;
+  }
+  unsigned row = 0, orow = ui;  // row offsets of direction k
+  int k = 0;
+  for (int sgm = 0; k < KL; ++sgm) {
+    const int kend = A.seg[sgm];
+    const bool ic = cs >= z, is = sn >= z;
+    const unsigned jlat = ic ? iS : iN, jlon = is ? iW : iE, jlat2 = RED ? (ic ? iS2 : iN2) : 0u;
+    const bool landlat = ic ? lS : lN, landlon = is ? lW : lE, landlat2 = RED && (ic ? lS2 : lN2);
+    const R wl = RED ? (ic ? wl1 : wl2) : one;
+    R in_lat[2], out_lat[2], in_lon[2], out_lon[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      in_lat[q] = ic ? L[q].kS : L[q].kN; out_lat[q] = ic ? L[q].kN : L[q].kS;
+      in_lon[q] = is ? L[q].kW : L[q].kE; out_lon[q] = is ? L[q].kE : L[q].kW;
+    }
+#pragma unroll UN
+    for (; k < kend; ++k) {
+      const bool wrap = k + 1 == KL;
+      const int kp = wrap ? 0 : k + 1;
+      const unsigned next = wrap ? 0u : row + st1;
+      const R snp = A.sinth[kp], csp = A.costh[kp];
+      R flat[2], flon[2], fkp[2], flat2[2] = {z, z};
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        fkp[q] = __ldg(fp[q] + (next + ui));
+        flat[q] = __ldg(fp[q] + (row + jlat));
+        flon[q] = __ldg(fp[q] + (row + jlon));
+        if (RED) flat2[q] = __ldg(fp[q] + (row + jlat2));
+        flat[q] = landlat ? z : flat[q];
+        flon[q] = landlon ? z : flon[q];
+        if (RED) flat2[q] = landlat2 ? z : flat2[q];
+      }
+      // direction-dependent terms common to both frequencies
+      const R sda = dabs(sn), cda = dabs(cs * A.DELPH0);
+      const R sp = SPH ? A.DELTH0 * (sn + snp) : z;
+      const R grad = TH ? snp * ddphi - csp * ddlam : z;
+      R dp_ = z, dpn_ = z, dle_ = z, dtc_ = z;  // deep spherical: without the frequency
+      if (SPH && !SH) {
+        dpn_ = cda * in_lat[0]; dle_ = sda * d0;
+        dp_ = L[0].drc * sp;
+        dtc_ = cda * out_lat[0] + dle_;
+        dtc_ = dtc_ + dmax(z, dp_) - L[0].mn;
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        Line<R>& l = L[q];
+        R sum, lat, lat2 = z, lon, th1 = z, th2 = z, mn = z;
+        if (SH) {
+          lat = cda * in_lat[q];
+          lon = sda * in_lon[q] * d0;
+          const R ol = sda * out_lon[q] * d0;
+          if (SPH) sum = (one - cda * out_lat[q]) - ol;
+          else sum = (one - ol) - cda * out_lat[q];
+          if (THETA) {
+            R d;
+            if (TH) {
+              const R thp = grad * l.tsi;
+              d = SPH ? l.drc * sp + (l.th + thp) * A.DELTHR : (l.th + thp) * A.DELTHR;
+              l.th = thp;
+            } else d = l.drc * sp;
+            const R mx = dmax(z, d);
+            mn = dmin(z, d);
+            sum = sum - mx + l.mn;
+            if (CNT) { const R qd = cd(d); th1 = -dmin(z, qd); th2 = dmax(z, qd); }
+            else { th1 = -mn; th2 = mx; }
+          }
+        } else if (SPH) {
+          const R g = gom[q];
+          mn = dmin(z, dp_);
+          lat = g * dpn_; lon = g * dle_;
+          th1 = -(g * mn); th2 = g * dmax(z, dp_);
+          sum = one - g * dtc_;
+          if (CNT) { th1 = cd(th1); th2 = cd(th2); }
+        } else {
+          const R g = gom[q];
+          lat = dabs(cs * A.DELPH0 * g); lon = dabs(sn * g) * d0;
+          sum = one - lon - lat;
+        }
+        if (RED && SPH) { lat2 = lat * (one - wl); lat = lat * wl; }
+        if (CNT) {
+          lat = cd(lat); lon = cd(lon);
+          if (RED) lat2 = cd(lat2);
+          sum = one - cd(one - sum);
+        }
+        R v = sum * l.fk + lat * flat[q] + lon * flon[q];
+        if (THETA) { v = v + th1 * fkp[q] + l.up; l.up = th2 * l.fk; }
+        if (RED) v = v + lat2 * flat2[q];
+        if (q == 0 || two) op[q][orow] = v;
+        l.fk = fkp[q]; l.mn = mn;
+      }
+      row = next; orow += st3;
+      sn = snp; cs = csp;
+    }
+  }
+}
+
+// The rows of n points from i of both planes, all directions, on their way to
+// L2: a thread per row, issued before the stencil's first load.  A thread keeps
+// only the loads of three directions in flight, which covers the latency of L2
+// but not that of DRAM.  Whole 16-byte granules: they hold valid data and so lie
+// in mapped pages.
+template <typename R>
+__device__ __forceinline__ void prefetch_rows(const R* __restrict__ f1, int ld1, int KL, int i, int n, int m, bool two) {
+  for (int t = threadIdx.x; t < (two ? 2 * KL : KL); t += blockDim.x) {
+    const int q = t >= KL ? 1 : 0;
+    const unsigned long long p = (unsigned long long)(f1 + (size_t)ld1 * ((size_t)KL * (m + q) + (t - q * KL)) + i);
+    const unsigned long long b = p & ~15ull, e = (p + (unsigned long long)n * sizeof(R) + 15) & ~15ull;
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(b), "r"((unsigned)(e - b)) : "memory");
   }
 }
 
 // Frequencies m0 + 2*blockIdx.y and the next one (if below m0 + mcount).
-template <typename R, int VAR, bool RED, bool REFRD>
-__global__ void __launch_bounds__(128) propags2_kernel(const __grid_constant__ PropArgs<R> A, const R* __restrict__ f1,
-                                                       int ld1, R* __restrict__ f3, int ld3, int m0, int mcount) {
-  const int i = A.i0 + blockIdx.x * blockDim.x + threadIdx.x;
+template <typename R, int VAR, bool RED, bool REFRD, bool CNT>
+__global__ void __launch_bounds__(128) propags_pair_kernel(const __grid_constant__ PropArgs<R> A, const R* __restrict__ f1,
+                                                           int ld1, R* __restrict__ f3, int ld3, int m0, int mcount) {
+  const int ib = A.i0 + blockIdx.x * blockDim.x, i = ib + threadIdx.x, q = 2 * blockIdx.y;
+  prefetch_rows(f1, ld1, A.KL, ib, min((int)blockDim.x, A.i1 - ib), m0 + q, q + 1 < mcount);
   if (i >= A.i1) return;
-  const int q = 2 * blockIdx.y;
-  propags_point2<R, VAR, RED, REFRD>(A, f1, ld1, f3, ld3, i, m0 + q, q + 1 < mcount);
+  propags_pair<R, VAR, RED, REFRD, CNT>(A, f1, ld1, f3, ld3, i, m0 + q, q + 1 < mcount);
 }
 
 // Batched form: every member of an ensemble (one coefficient family) in one
 // launch of BS-point CTAs.  CTA b belongs to member g with first[g] <= b <
-// first[g + 1] and covers frequency m and points ib*BS .. of that member; the
-// member's metadata block (direction tables included) is copied into shared
+// first[g + 1] and covers one frequency, or two of them where the pair stencil
+// applies (PropMember::pair), of BS points of that member; the member's metadata block (direction tables included) is copied into shared
 // memory first.
 template <typename R, int VAR, bool RED, bool REFRD, int BS>
 __global__ void __launch_bounds__(BS) propags_batch_kernel(const PropMember<R>* __restrict__ mem,
@@ -133,10 +314,21 @@ __global__ void __launch_bounds__(BS) propags_batch_kernel(const PropMember<R>* 
     for (int q = threadIdx.x; q < nw; q += BS) dst[q] = src[q];
   }
   __syncthreads();
-  const int lb = (int)blockIdx.x - first[g], m = lb / sm.nbi, ib = lb - m * sm.nbi;
-  const int i = sm.A.i0 + ib * BS + threadIdx.x;
+  const int lb = (int)blockIdx.x - first[g], r = lb / sm.nbi;
+  const int ib = sm.A.i0 + (lb - r * sm.nbi) * BS, i = ib + threadIdx.x;
+  if constexpr (!Site<R, VAR, RED, REFRD>::CUR) {
+    if (sm.pair) {
+      const int m = 2 * r;
+      const bool two = m + 1 < sm.A.ML;
+      prefetch_rows(sm.src, sm.ld, sm.A.KL, ib, min(BS, sm.A.i1 - ib), m, two);
+      if (i >= sm.A.i1) return;
+      if (sm.A.counter == 1) propags_pair<R, VAR, RED, REFRD, false>(sm.A, sm.src, sm.ld, sm.dst, sm.ld, i, m, two);
+      else propags_pair<R, VAR, RED, REFRD, true>(sm.A, sm.src, sm.ld, sm.dst, sm.ld, i, m, two);
+      return;
+    }
+  }
   if (i >= sm.A.i1) return;
-  propags_point<R, VAR, RED, REFRD>(sm.A, sm.src, sm.ld, sm.dst, sm.ld, i, m);
+  propags_point<R, VAR, RED, REFRD>(sm.A, sm.src, sm.ld, sm.dst, sm.ld, i, r);
 }
 
 // Transpose of one sub-step, thread per (sea point i, frequency m): every
@@ -252,12 +444,11 @@ cudaError_t dispatch(const PropArgs<R>& A, Args&&... args) {
 
 template <typename R, int V, bool RED, bool RD> struct PropLaunch {
   static cudaError_t run(const PropArgs<R>& A, const R* f1, int ld1, R* f3, int ld3, int m0, int mcount, cudaStream_t s) {
-    if constexpr (!var_current(V)) {
-      if (mcount >= 2) {
-        dim3 grid((A.i1 - A.i0 + 127) / 128, (mcount + 1) / 2);
-        propags2_kernel<R, V, RED, RD><<<grid, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
-        return cudaGetLastError();
-      }
+    if constexpr (!var_current(V)) if (propags_pairs(A, std::max(ld1, ld3))) {
+      const dim3 grid((A.i1 - A.i0 + 127) / 128, (mcount + 1) / 2);
+      if (A.counter == 1) propags_pair_kernel<R, V, RED, RD, false><<<grid, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
+      else propags_pair_kernel<R, V, RED, RD, true><<<grid, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
+      return cudaGetLastError();
     }
     dim3 grid((A.i1 - A.i0 + 127) / 128, mcount);
     propags_kernel<R, V, RED, RD><<<grid, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0);

@@ -35,6 +35,9 @@ template <typename R> struct PropArgs {
   // kernel parameter, so these are constant-bank reads (broadcast: every lane
   // of a warp reads the same direction), and every grid carries its own.
   R sinth[MAX_KL], costh[MAX_KL];
+  // Ends of the segments of directions within which neither SIN nor COS changes
+  // sign (seg[0] = 0: more than eight of them).
+  int seg[8];
 };
 
 }  // namespace wamgpu
