@@ -3,14 +3,18 @@
 // are functions of one sea point's spectrum and fields, so that an output
 // step reads NSEA x 40 values instead of downloading the spectrum.
 //
-// One thread integrates one sea point.  The spectrum FL3(IJ,K,M) has the sea
-// point fastest, so the 32 threads of a warp read 128 contiguous bytes of
-// every bin; the kernel reads the spectrum once (HBM-bound: KL*ML*4 bytes
-// per point in, 160 bytes out).  The direction sums of MEAN_DIRECTION and the
-// frequency sums of the other integrals are kept per thread in shared memory
-// (thread-fastest, conflict-free), and every sum runs in the reference's
-// order.  The unit is compiled without FMA contraction, so the results are
-// those of the reference's separate operations; only ATAN2 (current
+// A CTA of six warps integrates 32 sea points, lane = point.  The spectrum
+// FL3(IJ,K,M) has the sea point fastest, so a warp reads 128 contiguous bytes
+// of every bin.  The warps first take frequencies (the sums over directions),
+// then directions (the sums over frequencies), so that every sum is one
+// thread's loop in the reference's order with its loads in flight together; the
+// second reading comes from L2, where a CTA's 138 KB still lie.  The integrals
+// are then dealt out to the warps.  One thread per point, the direction sums in
+// shared memory, had 18 warps on an SM wait for one chain of loads each: 84k
+// points, 36x30, the parameters and the wind sea / swell split together 1275 us,
+// now 407 us (a reading of the spectrum from DRAM takes 56 us; each of the two
+// calls needs one).  The unit is compiled without FMA contraction, so the
+// results are those of the reference's separate operations; only ATAN2 (current
 // direction, mean direction) is the device library's.
 //
 // Routines (wam_interface_module.f90): TOTAL_ENERGY_B :1342-1410, FEMEAN
@@ -25,7 +29,8 @@ namespace wamgpu {
 
 namespace {
 
-constexpr int kOutThreads = 128;
+constexpr int kOutWarps = 6;
+static_assert(kOutWarps == 6, "the integrals are dealt out to six warps");
 
 template <typename R> struct OutConst {
   static constexpr R DEG = R(180.) / Phys<R>::PI;
@@ -47,237 +52,237 @@ __global__ void __launch_bounds__(256) ustar_max_kernel(const R* __restrict__ us
   if ((threadIdx.x & 31) == 0 && best) atomicMax(out, best);
 }
 
+// The integrals of one spectrum from its frequency sums Tm[m * 32] (directions
+// summed in order) and direction sums Tk[k * 32] (DFIM-weighted, frequencies in
+// order), in three independent parts for different warps.  TOTAL_ENERGY, FEMEAN
+// and TM1_TM2_PERIODS: Hs, TM, TM1, TM2 to the rows p0.. (p0 + 2..4).
+template <typename R, class Put>
+__device__ __forceinline__ void energy_part(const OutArgs<R>& a, const R* Tm, const Put& put, int phs, int ptm) {
+  const int ml = a.ML;
+  const R tail = Tm[(ml - 1) * 32];
+  R E = a.MO_TAIL * tail, FM = a.MM1_TAIL * tail, TM1 = a.MP1_TAIL * tail, TM2 = a.MP2_TAIL * tail;
+  for (int m = 0; m < ml; ++m) {
+    const R t = Tm[m * 32];
+    E = E + t * a.DFIM[m];
+    FM = FM + t * a.DFIMOFR[m];
+    TM1 = TM1 + t * a.DFIM_FR[m];
+    TM2 = TM2 + t * a.DFIM_FR2[m];
+  }
+  E = dmax(E, R(1.0E-12));
+  FM = E / dmax(FM, R(1.0E-12));
+  put(phs, R(4.) * sqrt(E));
+  put(ptm, R(1.) / FM);
+  put(ptm + 1, (E > R(1.0E-12)) ? E / TM1 : R(1.));
+  put(ptm + 2, (E > R(1.0E-12)) ? sqrt(E / TM2) : R(1.));
+}
+
+// PEAK_PERIOD: the first maximum of the frequency spectrum.
+template <typename R> __device__ __forceinline__ R peak_part(const OutArgs<R>& a, const R* Tm) {
+  int ip = 0;
+  R best = Tm[0];
+  for (int m = 1; m < a.ML; ++m) {
+    const R t = Tm[m * 32];
+    if (t > best) { best = t; ip = m; }
+  }
+  return ip == 0 ? R(1.) : R(1.) / a.FR[ip];
+}
+
+// MEAN_DIRECTION: direction and spread to the rows pd, pd + 1.
+template <typename R, class Put>
+__device__ __forceinline__ void direction_part(const OutArgs<R>& a, const R* Tk, const Put& put, int pd) {
+  using P_ = Phys<R>;
+  const R DEG = OutConst<R>::DEG;
+  R SI = 0, CI = 0, SP = 0;
+  for (int k = 0; k < a.KL; ++k) {
+    const R t = Tk[k * 32];
+    SI = SI + a.SINTH[k] * t;
+    CI = CI + a.COSTH[k] * t;
+    SP = SP + t;
+  }
+  {
+    const R ci = (CI == R(0.)) ? R(0.1E-30) : CI;
+    R thq = atan2(SI, ci);
+    if (thq < R(0.)) thq = thq + P_::ZPI;
+    if (thq > P_::ZPI - R(0.001)) thq = R(0.);
+    put(pd, orient(thq * DEG, a.from));
+  }
+  {
+    const R lim = R(0.1E-15);
+    const R ci = (dabs(CI) < lim) ? copysign(lim, CI) : CI;
+    const R si = (dabs(SI) < lim) ? copysign(lim, SI) : SI;
+    R sp = (dabs(SP) < lim) ? copysign(lim, SP) : SP;
+    sp = R(2.) * (R(1.) - sqrt(si * si + ci * ci) / sp);
+    sp = (sp <= R(0)) ? (sizeof(R) == 4 ? R(FLT_MIN) : R(DBL_MIN)) : sqrt(sp);  // TINY(1.)
+    put(pd + 1, sp * DEG);
+  }
+}
+
 template <typename R>
-__global__ void __launch_bounds__(kOutThreads) output_kernel(const __grid_constant__ OutArgs<R> a) {
+__global__ void __launch_bounds__(kOutWarps * 32) output_kernel(const __grid_constant__ OutArgs<R> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  R* sm = reinterpret_cast<R*>(smem_raw);
-  const int tid = threadIdx.x;
-  const int ij = blockIdx.x * kOutThreads + tid;
-  if (ij >= a.nsea) return;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int ij = min((int)blockIdx.x * 32 + lane, a.nsea - 1);
+  const bool real = (int)blockIdx.x * 32 + lane < a.nsea;
   const int kl = a.KL, ml = a.ML;
   using P_ = Phys<R>;
   const R DEG = OutConst<R>::DEG;
-  R* Tk = sm + tid;                       // [k * kOutThreads]: direction sums over frequency
-  R* Tm = sm + kl * kOutThreads + tid;    // [m * kOutThreads]: frequency spectrum (sum over directions)
-  for (int k = 0; k < kl; ++k) Tk[k * kOutThreads] = R(0);
+  R* Tk = reinterpret_cast<R*>(smem_raw) + lane;  // [k * 32]: direction sums over frequency
+  R* Tm = Tk + kl * 32;                           // [m * 32]: frequency spectrum (sum over directions)
+  R* DF = Tm + ml * 32 - lane;                    // DFIM
+  for (int m = threadIdx.x; m < ml; m += kOutWarps * 32) DF[m] = a.DFIM[m];
+  __syncthreads();
   const R* f = a.fl3 + ij;
-  for (int m = 0; m < ml; ++m) {
-    const R dfim = a.DFIM[m];
+  for (int m = w; m < ml; m += kOutWarps) {
+    const R* fm = f + (size_t)a.ld * kl * m;
     R s = R(0);
-    for (int k = 0; k < kl; ++k) {
-      const R v = __ldg(f + (size_t)a.ld * (k + (size_t)kl * m));
-      s = s + v;
-      Tk[k * kOutThreads] = Tk[k * kOutThreads] + v * dfim;
-    }
-    Tm[m * kOutThreads] = s;
+#pragma unroll 12
+    for (int k = 0; k < kl; ++k, fm += a.ld) s = s + __ldg(fm);
+    Tm[m * 32] = s;
   }
-  R U10 = a.u10[ij], UDIR = a.udir[ij], TAUW = a.tauw[ij];
-  R USTAR = a.ustar[ij], Z0 = a.z0[ij];
-  if (a.ustar_max && *a.ustar_max == 0ull) {
-    // IF (MAXVAL(USTAR(:)).EQ.0.) CALL AIRSEA (U10, TAUW, USTAR, Z0)
-    adj::airsea<R, R>(a.A, U10, TAUW, USTAR, Z0);
-    a.ustar[ij] = USTAR;
-    a.z0[ij] = Z0;
+  for (int k = w; k < kl; k += kOutWarps) {
+    const R* fk = f + (size_t)a.ld * k;
+    const size_t step = (size_t)a.ld * kl;
+    R t = R(0);
+#pragma unroll 10
+    for (int m = 0; m < ml; ++m, fk += step) t = t + __ldg(fk) * DF[m];
+    Tk[k * 32] = t;
   }
+  __syncthreads();
   R* out = a.block + ij;
-  auto put = [&](int p, R v) { out[(size_t)a.block_ld * (p - 1)] = v; };
-  const R tail = Tm[(ml - 1) * kOutThreads];
-  put(1, U10);
-  put(2, orient(DEG * UDIR, a.from));
-  put(3, USTAR);
-  const R TAU = USTAR * USTAR + R(0.0001);
-  put(4, TAU / (U10 * U10 + R(0.01)));
-  put(16, TAUW / (TAU * P_::ROAIR));
-  put(5, P_::G * Z0 / dmax(USTAR * USTAR, R(1.0E-6)));
-  put(6, a.shallow ? a.depth[ij] : R(999.));
-  const R cu = a.u ? a.u[ij] : R(0), cv = a.v ? a.v[ij] : R(0);
-  put(7, sqrt(cu * cu + cv * cv));
-  R cdir = orient(atan2(cu, cv) * DEG, a.from);
-  if (cdir < R(0.)) cdir = cdir + R(360.);
-  put(8, cdir);
-  // TOTAL_ENERGY, FEMEAN, TM1, TM2 and MEANSQS: frequency sums in order
-  R E = a.MO_TAIL * tail, FM = a.MM1_TAIL * tail, TM1 = a.MP1_TAIL * tail, TM2 = a.MP2_TAIL * tail;
-  R SM = R(1.0E-33);  // MAX(CONST2*TEMP(ML), EPSMIN) with CONST2 = 0.*LOG(FC/FS) = 0
-  for (int m = 0; m < ml; ++m) {
-    const R t = Tm[m * kOutThreads];
-    E = E + t * a.DFIM[m];
-    FM = FM + t * a.DFIMOFR[m];
-    TM1 = TM1 + t * a.DFIM_FR[m];
-    TM2 = TM2 + t * a.DFIM_FR2[m];
-    if (a.shallow) {
-      const R tk = __ldg(&a.TFAK[(a.indep[ij] - 1) + a.NDEPTH * m]);
-      SM = SM + a.DFIM[m] * (tk * tk) * t;
-    } else {
-      SM = SM + a.MSSFD[m] * t;
+  auto put = [&](int p, R v) { if (real) out[(size_t)a.block_ld * (p - 1)] = v; };
+  if (w == 0) {
+    energy_part(a, Tm, put, 9, 11);
+  } else if (w == 1) {
+    put(10, peak_part(a, Tm));
+  } else if (w == 2) {
+    direction_part(a, Tk, put, 14);
+  } else if (w == 3) {  // MEANSQS
+    R SM = R(1.0E-33);  // MAX(CONST2*TEMP(ML), EPSMIN) with CONST2 = 0.*LOG(FC/FS) = 0
+    const int jd = a.shallow ? a.indep[ij] - 1 : 0;
+    for (int m = 0; m < ml; ++m) {
+      const R t = Tm[m * 32];
+      if (a.shallow) {
+        const R tk = __ldg(&a.TFAK[jd + a.NDEPTH * m]);
+        SM = SM + a.DFIM[m] * (tk * tk) * t;
+      } else {
+        SM = SM + a.MSSFD[m] * t;
+      }
     }
+    put(40, SM);
+  } else if (w == 4) {
+    R U10 = a.u10[ij], UDIR = a.udir[ij], TAUW = a.tauw[ij];
+    R USTAR = a.ustar[ij], Z0 = a.z0[ij];
+    if (a.ustar_max && *a.ustar_max == 0ull) {
+      // IF (MAXVAL(USTAR(:)).EQ.0.) CALL AIRSEA (U10, TAUW, USTAR, Z0)
+      adj::airsea<R, R>(a.A, U10, TAUW, USTAR, Z0);
+      if (real) { a.ustar[ij] = USTAR; a.z0[ij] = Z0; }
+    }
+    put(1, U10);
+    put(2, orient(DEG * UDIR, a.from));
+    put(3, USTAR);
+    const R TAU = USTAR * USTAR + R(0.0001);
+    put(4, TAU / (U10 * U10 + R(0.01)));
+    put(16, TAUW / (TAU * P_::ROAIR));
+    put(5, P_::G * Z0 / dmax(USTAR * USTAR, R(1.0E-6)));
+    put(32, Z0);
+  } else {
+    put(6, a.shallow ? a.depth[ij] : R(999.));
+    const R cu = a.u ? a.u[ij] : R(0), cv = a.v ? a.v[ij] : R(0);
+    put(7, sqrt(cu * cu + cv * cv));
+    R cdir = orient(atan2(cu, cv) * DEG, a.from);
+    if (cdir < R(0.)) cdir = cdir + R(360.);
+    put(8, cdir);
+    // parameters that are not computed stay 0
+    for (int p = 17; p < 40; ++p)
+      if (p != 32) put(p, R(0));
   }
-  E = dmax(E, R(1.0E-12));
-  FM = E / dmax(FM, R(1.0E-12));
-  put(11, R(1.) / FM);
-  put(40, SM);
-  put(12, (E > R(1.0E-12)) ? E / TM1 : R(1.));
-  put(13, (E > R(1.0E-12)) ? sqrt(E / TM2) : R(1.));
-  put(9, R(4.) * sqrt(E));
-  // PEAK_PERIOD: the first maximum of the frequency spectrum
-  int ip = 0;
-  R best = Tm[0];
-  for (int m = 1; m < ml; ++m) {
-    const R t = Tm[m * kOutThreads];
-    if (t > best) { best = t; ip = m; }
-  }
-  put(10, ip == 0 ? R(1.) : R(1.) / a.FR[ip]);
-  // MEAN_DIRECTION: THQ and SPREAD
-  R SI = 0, CI = 0, SP = 0;
-  for (int k = 0; k < kl; ++k) {
-    const R t = Tk[k * kOutThreads];
-    SI = SI + a.SINTH[k] * t;
-    CI = CI + a.COSTH[k] * t;
-    SP = SP + t;
-  }
-  {
-    const R ci = (CI == R(0.)) ? R(0.1E-30) : CI;
-    R thq = atan2(SI, ci);
-    if (thq < R(0.)) thq = thq + P_::ZPI;
-    if (thq > P_::ZPI - R(0.001)) thq = R(0.);
-    put(14, orient(thq * DEG, a.from));
-  }
-  {
-    const R lim = R(0.1E-15);
-    const R ci = (dabs(CI) < lim) ? copysign(lim, CI) : CI;
-    const R si = (dabs(SI) < lim) ? copysign(lim, SI) : SI;
-    R sp = (dabs(SP) < lim) ? copysign(lim, SP) : SP;
-    sp = R(2.) * (R(1.) - sqrt(si * si + ci * ci) / sp);
-    sp = (sp <= R(0)) ? (sizeof(R) == 4 ? R(FLT_MIN) : R(DBL_MIN)) : sqrt(sp);  // TINY(1.)
-    put(15, sp * DEG);
-  }
-  put(32, Z0);
 }
-
-// The integrals COMPUTE_OUTPUT_PARAMETER and SWELL_SEPARATION take of one
-// spectrum, from its frequency sums Tm[m * st] (directions summed in order)
-// and direction sums Tk[k * st] (DFIM-weighted, frequencies in order):
-// TOTAL_ENERGY, FEMEAN, TM1_TM2_PERIODS, PEAK_PERIOD, MEAN_DIRECTION, in the
-// statement order of the parameters 9-15 above.
-template <typename R> struct SpecInt { R E, TM, TM1, TM2, TP, THQ, SPREAD; };
-template <typename R>
-__device__ SpecInt<R> spec_integrals(const OutArgs<R>& a, const R* Tk, const R* Tm, int st) {
-  using P_ = Phys<R>;
-  const int kl = a.KL, ml = a.ML;
-  const R DEG = OutConst<R>::DEG;
-  SpecInt<R> o;
-  const R tail = Tm[(ml - 1) * st];
-  R E = a.MO_TAIL * tail, FM = a.MM1_TAIL * tail, TM1 = a.MP1_TAIL * tail, TM2 = a.MP2_TAIL * tail;
-  for (int m = 0; m < ml; ++m) {
-    const R t = Tm[m * st];
-    E = E + t * a.DFIM[m];
-    FM = FM + t * a.DFIMOFR[m];
-    TM1 = TM1 + t * a.DFIM_FR[m];
-    TM2 = TM2 + t * a.DFIM_FR2[m];
-  }
-  E = dmax(E, R(1.0E-12));
-  FM = E / dmax(FM, R(1.0E-12));
-  o.E = E;
-  o.TM = R(1.) / FM;
-  o.TM1 = (E > R(1.0E-12)) ? E / TM1 : R(1.);
-  o.TM2 = (E > R(1.0E-12)) ? sqrt(E / TM2) : R(1.);
-  int ip = 0;
-  R best = Tm[0];
-  for (int m = 1; m < ml; ++m) {
-    const R t = Tm[m * st];
-    if (t > best) { best = t; ip = m; }
-  }
-  o.TP = ip == 0 ? R(1.) : R(1.) / a.FR[ip];
-  R SI = 0, CI = 0, SP = 0;
-  for (int k = 0; k < kl; ++k) {
-    const R t = Tk[k * st];
-    SI = SI + a.SINTH[k] * t;
-    CI = CI + a.COSTH[k] * t;
-    SP = SP + t;
-  }
-  {
-    const R ci = (CI == R(0.)) ? R(0.1E-30) : CI;
-    R thq = atan2(SI, ci);
-    if (thq < R(0.)) thq = thq + P_::ZPI;
-    if (thq > P_::ZPI - R(0.001)) thq = R(0.);
-    o.THQ = orient(thq * DEG, a.from);
-  }
-  {
-    const R lim = R(0.1E-15);
-    const R ci = (dabs(CI) < lim) ? copysign(lim, CI) : CI;
-    const R si = (dabs(SI) < lim) ? copysign(lim, SI) : SI;
-    R sp = (dabs(SP) < lim) ? copysign(lim, SP) : SP;
-    sp = R(2.) * (R(1.) - sqrt(si * si + ci * ci) / sp);
-    sp = (sp <= R(0)) ? (sizeof(R) == 4 ? R(FLT_MIN) : R(DBL_MIN)) : sqrt(sp);  // TINY(1.)
-    o.SPREAD = sp * DEG;
-  }
-  return o;
-}
-
-constexpr int kSwThreads = 64;
 
 // SWELL_SEPARATION (wam_swell_module.f90:106-350) without the partitioning
-// (parameters 41-49).  One thread per sea point walks the directions: a bin
-// is swell where FRIC/C(M) * 1.2*USTAR*COS(TH(K)-UDIR) < 1, its swell value
-// MAX(F, EPSMIN) there and 0 elsewhere, its wind-sea value F minus that.
-// The cosine is the correctly rounded single-precision value (the oracle
-// forms it the same way, so both split every bin alike).  The frequency sums
-// of both spectra still add their directions in order, the direction sums
+// (parameters 41-49).  A bin is swell where FRIC/C(M) * 1.2*USTAR*COS(TH(K)-UDIR)
+// < 1, its swell value MAX(F, EPSMIN) there and 0 elsewhere, its wind-sea value
+// F minus that.  The cosine is the correctly rounded single-precision value (the
+// oracle forms it the same way, so both split every bin alike).  The frequency
+// sums of both spectra still add their directions in order, the direction sums
 // their frequencies in order.  Parameters 17-23 (wind sea) and 25-31 (swell):
 // Hs, peak period, mean period, TM1, TM2, mean direction, spread.
 template <typename R>
-__global__ void __launch_bounds__(kSwThreads) swell_kernel(const __grid_constant__ OutArgs<R> a) {
+__global__ void __launch_bounds__(kOutWarps * 32) swell_kernel(const __grid_constant__ OutArgs<R> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  R* sm = reinterpret_cast<R*>(smem_raw);
-  const int tid = threadIdx.x;
-  const int ij = blockIdx.x * kSwThreads + tid;
-  if (ij >= a.nsea) return;
-  const int kl = a.KL, ml = a.ML, st = kSwThreads;
-  R* Tk1 = sm + tid;                      // swell direction sums
-  R* Tk4 = Tk1 + kl * st;                 // wind-sea direction sums
-  R* Tm1 = Tk4 + kl * st;                 // swell frequency sums
-  R* Tm4 = Tm1 + ml * st;                 // wind-sea frequency sums
-  for (int m = 0; m < ml; ++m) { Tm1[m * st] = R(0); Tm4[m * st] = R(0); }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int ij = min((int)blockIdx.x * 32 + lane, a.nsea - 1);
+  const bool real = (int)blockIdx.x * 32 + lane < a.nsea;
+  const int kl = a.KL, ml = a.ML;
+  R* Tk1 = reinterpret_cast<R*>(smem_raw) + lane;  // swell direction sums
+  R* Tk4 = Tk1 + kl * 32;                          // wind-sea direction sums
+  R* Tm1 = Tk4 + kl * 32;                          // swell frequency sums
+  R* Tm4 = Tm1 + ml * 32;                          // wind-sea frequency sums
+  R* FP = Tm4 + ml * 32;                           // 1.2*USTAR*COS(TH(K)-UDIR)
+  R* CM = FP + kl * 32 - lane;                     // FRIC/C(M)
   const R FRIC = R(28.), EPSMIN = R(0.1E-32);
   const R us = a.ustar[ij], ud = a.udir[ij];
+  for (int k = w; k < kl; k += kOutWarps) FP[k * 32] = R(1.2) * us * crcos(a.TH[k] - ud);
+  R* DF = CM + ml;                                 // DFIM
+  for (int m = threadIdx.x; m < ml; m += kOutWarps * 32) { CM[m] = FRIC / a.C[m]; DF[m] = a.DFIM[m]; }
+  __syncthreads();
   const R* f = a.fl3 + ij;
-  for (int k = 0; k < kl; ++k) {
-    const R flpp = R(1.2) * us * crcos(a.TH[k] - ud);
-    R t1 = R(0), t4 = R(0);
-    for (int m = 0; m < ml; ++m) {
-      const R v = __ldg(f + (size_t)a.ld * (k + (size_t)kl * m));
-      const R cm = FRIC / a.C[m];
-      const R f1 = (cm * flpp < R(1.0)) ? dmax(v, EPSMIN) : R(0.);
-      const R f4 = v - f1;
-      Tm1[m * st] = Tm1[m * st] + f1;
-      Tm4[m * st] = Tm4[m * st] + f4;
-      t1 = t1 + f1 * a.DFIM[m];
-      t4 = t4 + f4 * a.DFIM[m];
+  for (int m = w; m < ml; m += kOutWarps) {
+    const R* fm = f + (size_t)a.ld * kl * m;
+    const R cm = CM[m];
+    R s1 = R(0), s4 = R(0);
+#pragma unroll 12
+    for (int k = 0; k < kl; ++k, fm += a.ld) {
+      const R v = __ldg(fm);
+      const R f1 = (cm * FP[k * 32] < R(1.0)) ? dmax(v, EPSMIN) : R(0.);
+      s1 = s1 + f1;
+      s4 = s4 + (v - f1);
     }
-    Tk1[k * st] = t1;
-    Tk4[k * st] = t4;
+    Tm1[m * 32] = s1;
+    Tm4[m * 32] = s4;
   }
+  for (int k = w; k < kl; k += kOutWarps) {
+    const R* fk = f + (size_t)a.ld * k;
+    const size_t step = (size_t)a.ld * kl;
+    const R flpp = FP[k * 32];
+    R t1 = R(0), t4 = R(0);
+#pragma unroll 10
+    for (int m = 0; m < ml; ++m, fk += step) {
+      const R v = __ldg(fk), df = DF[m];
+      const R f1 = (CM[m] * flpp < R(1.0)) ? dmax(v, EPSMIN) : R(0.);
+      t1 = t1 + f1 * df;
+      t4 = t4 + (v - f1) * df;
+    }
+    Tk1[k * 32] = t1;
+    Tk4[k * 32] = t4;
+  }
+  __syncthreads();
   R* out = a.block + ij;
-  auto put = [&](int p, R v) { out[(size_t)a.block_ld * (p - 1)] = v; };
-  const SpecInt<R> ws = spec_integrals(a, Tk4, Tm4, st), sw = spec_integrals(a, Tk1, Tm1, st);
-  put(17, R(4.) * sqrt(ws.E)); put(18, ws.TP); put(19, ws.TM); put(20, ws.TM1); put(21, ws.TM2);
-  put(22, ws.THQ); put(23, ws.SPREAD);
-  put(25, R(4.) * sqrt(sw.E)); put(26, sw.TP); put(27, sw.TM); put(28, sw.TM1); put(29, sw.TM2);
-  put(30, sw.THQ); put(31, sw.SPREAD);
+  auto put = [&](int p, R v) { if (real) out[(size_t)a.block_ld * (p - 1)] = v; };
+  // even warps the wind sea, odd ones the swell
+  const bool swell = w & 1;
+  const R* Tm = swell ? Tm1 : Tm4;
+  const int p = swell ? 25 : 17;
+  if (w < 2) energy_part(a, Tm, put, p, p + 2);
+  else if (w < 4) put(p + 1, peak_part(a, Tm));
+  else direction_part(a, swell ? Tk1 : Tk4, put, p + 5);
 }
+
+template <typename R> size_t output_smem(int KL, int ML) { return (size_t)(32 * (KL + ML) + ML) * sizeof(R); }
+template <typename R> size_t swell_smem(int KL, int ML) { return (size_t)(32 * (3 * KL + 2 * ML) + 2 * ML) * sizeof(R); }
 
 }  // namespace
 
 template <typename R> cudaError_t launch_swell(const OutArgs<R>& a, cudaStream_t s) {
   if (a.nsea == 0) return cudaSuccess;
-  const size_t smem = (size_t)kSwThreads * 2 * (a.KL + a.ML) * sizeof(R);
+  const size_t smem = swell_smem<R>(a.KL, a.ML);
   static bool raised[2] = {false, false};
   if (smem > 48 * 1024 && !raised[sizeof(R) == 8]) {
     cudaError_t e = cudaFuncSetAttribute(swell_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)((size_t)kSwThreads * 2 * (MAX_KL + MAX_ML) * sizeof(R)));
+                                         (int)swell_smem<R>(MAX_KL, MAX_ML));
     if (e != cudaSuccess) return e;
     raised[sizeof(R) == 8] = true;
   }
-  swell_kernel<R><<<(a.nsea + kSwThreads - 1) / kSwThreads, kSwThreads, smem, s>>>(a);
+  swell_kernel<R><<<(a.nsea + 31) / 32, kOutWarps * 32, smem, s>>>(a);
   return cudaGetLastError();
 }
 template cudaError_t launch_swell<float>(const OutArgs<float>&, cudaStream_t);
@@ -405,8 +410,6 @@ template cudaError_t launch_restart_scatter<float>(const float*, int, const int*
 template cudaError_t launch_restart_scatter<double>(const float*, int, const int*, int, int, double*, size_t,
                                                     cudaStream_t);
 
-template <typename R> size_t output_smem_bytes(int KL, int ML) { return (size_t)kOutThreads * (KL + ML) * sizeof(R); }
-
 template <typename R> cudaError_t launch_output(const OutArgs<R>& a, unsigned long long* ustar_max, cudaStream_t s) {
   if (a.nsea == 0) return cudaSuccess;
   OutArgs<R> b = a;
@@ -417,21 +420,19 @@ template <typename R> cudaError_t launch_output(const OutArgs<R>& a, unsigned lo
     ustar_max_kernel<R><<<148, 256, 0, s>>>(a.ustar, a.nsea, ustar_max);
     b.ustar_max = ustar_max;
   }
-  const size_t smem = output_smem_bytes<R>(a.KL, a.ML);
+  const size_t smem = output_smem<R>(a.KL, a.ML);
   static bool raised[2] = {false, false};
   if (smem > 48 * 1024 && !raised[sizeof(R) == 8]) {
     cudaError_t e = cudaFuncSetAttribute(output_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)output_smem_bytes<R>(MAX_KL, MAX_ML));
+                                         (int)output_smem<R>(MAX_KL, MAX_ML));
     if (e != cudaSuccess) return e;
     raised[sizeof(R) == 8] = true;
   }
-  output_kernel<R><<<(a.nsea + kOutThreads - 1) / kOutThreads, kOutThreads, smem, s>>>(b);
+  output_kernel<R><<<(a.nsea + 31) / 32, kOutWarps * 32, smem, s>>>(b);
   return cudaGetLastError();
 }
 
 template cudaError_t launch_output<float>(const OutArgs<float>&, unsigned long long*, cudaStream_t);
 template cudaError_t launch_output<double>(const OutArgs<double>&, unsigned long long*, cudaStream_t);
-template size_t output_smem_bytes<float>(int, int);
-template size_t output_smem_bytes<double>(int, int);
 
 }  // namespace wamgpu
