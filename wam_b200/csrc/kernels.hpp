@@ -75,11 +75,10 @@ template <typename R> struct PropMember {
   int ld, nbi;
   int pair;  // two frequencies per CTA (propags_pairs)
 };
-// Whether a sub-step takes two frequencies per thread: variants without
-// currents, 32-bit offsets in a plane, at most eight segments of directions.
-bool propags_planes_independent(int variant);
+// Whether a sub-step takes two frequencies per thread: 32-bit offsets in a plane,
+// and without currents at most eight segments of directions.
 template <typename R> bool propags_pairs(const PropArgs<R>& A, int ld) {
-  return propags_planes_independent(A.variant) && A.seg[0] > 0 && (size_t)ld * A.KL < (size_t(1) << 31);
+  return (A.seg[0] > 0 || !propags_planes_independent(A.variant)) && (size_t)ld * A.KL < (size_t(1) << 31);
 }
 // All members of one coefficient family (variant, reduced grid, depth
 // refraction taken from `family`) in one launch of bs-point CTAs (128 or 256);

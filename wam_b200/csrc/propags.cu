@@ -5,7 +5,8 @@
 
 namespace wamgpu {
 
-// One thread per (sea point i, frequency m) walking the directions.
+// One thread per (sea point i, frequency m) walking the directions: what the
+// pair stencils below do not take (propags_pairs).
 template <typename R, int VAR, bool RED, bool REFRD>
 __device__ __forceinline__ void propags_point(const PropArgs<R>& A, const R* __restrict__ f1, int ld1,
                                               R* __restrict__ f3, int ld3, int i, int m) {
@@ -265,6 +266,192 @@ __device__ __forceinline__ void propags_pair(const PropArgs<R>& A, const R* __re
   }
 }
 
+// What one frequency of a point carries with currents.
+template <typename R> struct CurLine {
+  R cg, cgS, cgN, cgW, cgE, cgS1, cgN1, tsi;
+  R fk;  // F(k)
+  R mn;  // negative part of DTM
+  R up;  // positive part of DTM (over COUNTER) times F(k-1)
+  R th;  // THDD(k)
+};
+
+// The stencil for the variants with currents, two frequencies m, m+1 of one sea
+// point per thread.  Issue-bound like the one above, and by the same means: one
+// boundary term serves direction k as DTP and k+1 as DTM; likewise one boundary
+// term in frequency serves m as DOP and m+1 as DOM, so that two frequencies take
+// three of them (from SIDC of m-1 .. m+2) instead of four; the direction's part
+// of THDD and SIDC (products of SIN and COS with the current gradients) is formed
+// once for both; F of one frequency is the other's neighbour in frequency; the
+// quotients by 1.1 and by COUNTER are exact scaled Markstein quotients.  The
+// expressions are those of Site::coef_w, so the results have the same bits.
+// The frequency pairs of a block of points run next to each other, so that the
+// planes m-1 and m+2, which other CTAs own, come from L2 on any grid.  A call on
+// 47k points, 36x30, COUNTER = 1, with its copy of the spectrum: 578 us by the
+// one-frequency kernel, 377 us.
+template <typename R, int VAR, bool RED, bool REFRD, bool CNT>
+__device__ __forceinline__ void propags_pair_cur(const PropArgs<R>& A, const R* __restrict__ f1, int ld1,
+                                                 R* __restrict__ f3, int ld3, int i, int m, bool two) {
+  using S = Site<R, VAR, RED, REFRD>;
+  static_assert(S::CUR, "for the variants with currents");
+  constexpr bool SH = S::SH, SPH = S::SPH;
+  const int KL = A.KL, mb = min(m + 1, A.ML - 1), mlo = max(m - 1, 0), mhi = two ? min(m + 2, A.ML - 1) : mb;
+  const R one = R(1.), z = R(0.);
+  unsigned iS, iN, iW, iE, iS2 = 0, iN2 = 0;  // neighbours' indices, the point's own for land
+  bool lS, lN, lW, lE, lS2 = false, lN2 = false;
+  R wl1 = one, wl2 = one, d0, dr, ps, pn, ddphi = z, ddlam = z, duphi, dulam, dvphi, dvlam;
+  R u0, uW, uE, v0, vS, vN, vS1 = z, vN1 = z;
+  R scg[4], stt[4], stk[4], sdf[3];  // SIDC's factors of m-1 .. m+2, DELFR0/FR of the three boundaries
+  CurLine<R> L[2];
+  {
+    auto nb = [&](int p1, unsigned& idx, bool& land) { land = p1 == 0; idx = land ? (unsigned)i : (unsigned)(p1 - 1); };
+    const S sa(A, i, m), sb(A, i, mb);
+    nb(sa.s0, iS, lS); nb(sa.n0, iN, lN); nb(sa.w0, iW, lW); nb(sa.e0, iE, lE);
+    if (RED) { nb(sa.s1, iS2, lS2); nb(sa.n1, iN2, lN2); wl1 = sa.wl1; wl2 = sa.wl2; vS1 = sa.vS1; vN1 = sa.vN1; }
+    d0 = sa.d0; dr = sa.dr; ps = sa.ps; pn = sa.pn;
+    duphi = sa.duphi; dulam = sa.dulam; dvphi = sa.dvphi; dvlam = sa.dvlam;
+    u0 = sa.u0; uW = sa.uW; uE = sa.uE; v0 = sa.v0; vS = sa.vS; vN = sa.vN;
+    if (SH) {
+      ddphi = sa.ddphi; ddlam = sa.ddlam;
+      scg[0] = sa.cgM; stt[0] = sa.tempc * sa.tsiM; stk[0] = sa.tfkM;
+      scg[1] = sa.cg; stt[1] = sa.tempc * sa.tsi; stk[1] = sa.tfk;
+      scg[2] = sb.cg; stt[2] = sa.tempc * sb.tsi; stk[2] = sb.tfk;
+      scg[3] = sb.cgP; stt[3] = sa.tempc * sb.tsiP; stk[3] = sb.tfkP;
+      sdf[0] = sa.dfm; sdf[1] = sa.dfp; sdf[2] = sb.dfp;
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const S& s = q ? sb : sa;
+      CurLine<R>& l = L[q];
+      if (SH) {
+        l.cg = s.cg; l.cgS = s.cgS; l.cgN = s.cgN; l.cgW = s.cgW; l.cgE = s.cgE; l.tsi = s.tsi;
+        l.cgS1 = s.cgS1; l.cgN1 = s.cgN1;
+      } else {
+        l.cg = l.cgS = l.cgN = l.cgW = l.cgE = l.cgS1 = l.cgN1 = s.gom; l.tsi = z;
+      }
+    }
+  }
+  const CounterDiv<R> cd(CNT ? A.rcounter : one), c11(R(1.1));
+  const size_t plane = (size_t)ld1 * KL;
+  const R* fp[2] = {f1 + plane * m, f1 + plane * mb};
+  const R *flo = f1 + plane * mlo, *fhi = f1 + plane * mhi;
+  R* op[2] = {f3 + (size_t)ld3 * KL * m, f3 + (size_t)ld3 * KL * mb};
+  const unsigned ui = (unsigned)i, st1 = (unsigned)ld1, st3 = (unsigned)ld3;
+  auto thdc = [&](R ss, R sc, R cc) { return ss * duphi + sc * dvphi - sc * dulam - cc * dvlam; };
+  // boundary in direction between k and k+1 of a frequency: sines, THDD of both
+  auto dbound = [&](const CurLine<R>& l, R sp, R spd, R t0, R tp) {
+    if (!SPH) return (t0 + tp) * A.DELTHR;
+    if (SH) return spd * l.cg + (t0 + tp) * A.DELTHR;
+    return sp * l.cg * dr + (t0 + tp) * A.DELTHR;
+  };
+  R sn = A.sinth[0], cs = A.costh[0];
+  R ss = sn * sn, sc = sn * cs, cc = cs * cs;
+  {
+    const R snl = A.sinth[KL - 1], csl = A.costh[KL - 1];
+    const R sp = A.DELTH0 * (sn + snl), spd = sp * dr;
+    const R t0 = thdc(ss, sc, cc), tl = thdc(snl * snl, snl * csl, csl * csl);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      CurLine<R>& l = L[q];
+      const R fl = __ldg(fp[q] + st1 * (unsigned)(KL - 1) + ui);
+      l.fk = __ldg(fp[q] + ui);
+      l.th = SH ? (sn * ddphi - cs * ddlam) * l.tsi + t0 : t0;
+      const R thm = SH ? (snl * ddphi - csl * ddlam) * l.tsi + tl : tl;
+      const R d = dbound(l, sp, spd, l.th, thm);
+      l.mn = dmin(z, d);
+      R th2 = dmax(z, d);
+      if (CNT) th2 = cd(th2);
+      l.up = th2 * fl;
+    }
+  }
+  unsigned row = 0, orow = ui;
+#pragma unroll 2
+  for (int k = 0; k < KL; ++k) {
+    const bool wrap = k + 1 == KL;
+    const int kp = wrap ? 0 : k + 1;
+    const unsigned next = wrap ? 0u : row + st1;
+    R fS[2], fN[2], fW[2], fE[2], fkp[2], fS2[2] = {z, z}, fN2[2] = {z, z};
+    const R fm1 = __ldg(flo + (row + ui)), fp2 = __ldg(fhi + (row + ui));
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      fkp[q] = __ldg(fp[q] + (next + ui));
+      fN[q] = __ldg(fp[q] + (row + iN)); fS[q] = __ldg(fp[q] + (row + iS));
+      fE[q] = __ldg(fp[q] + (row + iE)); fW[q] = __ldg(fp[q] + (row + iW));
+      if (RED) { fN2[q] = __ldg(fp[q] + (row + iN2)); fS2[q] = __ldg(fp[q] + (row + iS2)); }
+      fN[q] = lN ? z : fN[q]; fS[q] = lS ? z : fS[q]; fE[q] = lE ? z : fE[q]; fW[q] = lW ? z : fW[q];
+      if (RED) { fN2[q] = lN2 ? z : fN2[q]; fS2[q] = lS2 ? z : fS2[q]; }
+    }
+    const R snp = A.sinth[kp], csp = A.costh[kp];
+    // frequency shift: SIDC without the frequency, then the three boundaries
+    const R b = -(sc * duphi) - cc * dvphi - ss * dulam - sc * dvlam;
+    R g[3];
+    if (SH) {
+      R sv[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) sv[q] = (b * scg[q] + stt[q]) * stk[q];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) g[q] = (sv[q] + sv[q + 1]) * sdf[q];
+    } else {
+      g[0] = g[1] = g[2] = b * A.DELFR0;
+    }
+    const R ssp = snp * snp, scp = snp * csp, ccp = csp * csp;
+    const R tcp = thdc(ssp, scp, ccp), grad = SH ? snp * ddphi - csp * ddlam : z;
+    const R sp = SPH ? A.DELTH0 * (sn + snp) : z, spd = SPH && SH ? sp * dr : z;
+    R v[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      CurLine<R>& l = L[q];
+      const R w1 = u0 + sn * l.cg, w2 = (v0 + cs * l.cg) * A.DELPH0;
+      const R dlw = (w1 + (uW + sn * l.cgW)) * d0, dle = (w1 + (uE + sn * l.cgE)) * d0;
+      R dtc = one - dmax(z, dle) + dmin(z, dlw);
+      R lon1 = dmax(z, dlw), lon2 = -dmin(z, dle), lat11, lat12 = z, lat21, lat22 = z;
+      auto wok2 = [&](R vv, R cgv) { return (vv + cs * cgv) * A.DELPH0; };
+      if (!(SPH && RED)) {
+        const R dps = SPH ? w2 + ps * wok2(vS, l.cgS) : w2 + wok2(vS, l.cgS);
+        const R dpn = SPH ? w2 + pn * wok2(vN, l.cgN) : w2 + wok2(vN, l.cgN);
+        dtc = dtc - dmax(z, dpn) + dmin(z, dps);
+        lat11 = dmax(z, dps); lat21 = -dmin(z, dpn);
+      } else {
+        R dps, dps2, dpn, dpn2;
+        if (SH) {
+          dps = w2 + ps * (wl1 * wok2(vS, l.cgS) + (one - wl1) * wok2(vS1, l.cgS1));
+          dps2 = dps * (one - wl1); dps = dps * wl1;
+          dpn = w2 + pn * (wl2 * wok2(vN, l.cgN) + (one - wl2) * wok2(vN1, l.cgN1));
+          dpn2 = dpn * (one - wl2); dpn = dpn * wl2;
+        } else {
+          dps = (w2 + wok2(vS, l.cgS) * ps) * wl1; dps2 = (w2 + wok2(vS1, l.cgS1) * ps) * (one - wl1);
+          dpn = (w2 + wok2(vN, l.cgN) * pn) * wl2; dpn2 = (w2 + wok2(vN1, l.cgN1) * pn) * (one - wl2);
+        }
+        dtc = dtc - dmax(z, dpn) - dmax(z, dpn2) + dmin(z, dps) + dmin(z, dps2);
+        lat11 = dmax(z, dps); lat12 = dmax(z, dps2); lat21 = -dmin(z, dpn); lat22 = -dmin(z, dpn2);
+      }
+      const R thp = SH ? grad * l.tsi + tcp : tcp;
+      const R d = dbound(l, sp, spd, l.th, thp);
+      const R mx = dmax(z, d), mn = dmin(z, d);
+      dtc = dtc - mx + l.mn;
+      R th1 = -mn, th2 = mx;
+      R sg1 = c11(-dmin(z, g[q + 1])), sg2 = dmax(z, g[q]) * R(1.1);
+      R sum = SH ? dtc - dmax(z, g[q + 1]) + dmin(z, g[q]) : dtc - dabs(g[0]);
+      if (CNT) {
+        lat11 = cd(lat11); lat21 = cd(lat21); lon1 = cd(lon1); lon2 = cd(lon2);
+        if (RED) { lat12 = cd(lat12); lat22 = cd(lat22); }
+        th1 = cd(th1); th2 = cd(th2); sg1 = cd(sg1); sg2 = cd(sg2);
+        sum = one - cd(one - sum);
+      }
+      const R fmp = q ? fp2 : L[1].fk, fmm = q ? L[0].fk : fm1;
+      v[q] = sum * l.fk + lat21 * fN[q] + lat11 * fS[q] + lon2 * fE[q] + lon1 * fW[q] + th1 * fkp[q] + l.up + sg1 * fmp +
+             sg2 * fmm;
+      if (RED) v[q] = v[q] + lat22 * fN2[q] + lat12 * fS2[q];
+      l.up = th2 * l.fk;
+      l.mn = mn; l.th = thp;
+    }
+    op[0][orow] = v[0];
+    if (two) op[1][orow] = v[1];
+    L[0].fk = fkp[0]; L[1].fk = fkp[1];
+    row = next; orow += st3;
+    sn = snp; cs = csp; ss = ssp; sc = scp; cc = ccp;
+  }
+}
+
 // The rows of n points from i of both planes, all directions, on their way to
 // L2: a thread per row, issued before the stencil's first load.  A thread keeps
 // only the loads of three directions in flight, which covers the latency of L2
@@ -288,6 +475,17 @@ __global__ void __launch_bounds__(128) propags_pair_kernel(const __grid_constant
   prefetch_rows(f1, ld1, A.KL, ib, min((int)blockDim.x, A.i1 - ib), m0 + q, q + 1 < mcount);
   if (i >= A.i1) return;
   propags_pair<R, VAR, RED, REFRD, CNT>(A, f1, ld1, f3, ld3, i, m0 + q, q + 1 < mcount);
+}
+
+template <typename R, int VAR, bool RED, bool REFRD, bool CNT>
+__global__ void __launch_bounds__(128) propags_pair_cur_kernel(const __grid_constant__ PropArgs<R> A,
+                                                               const R* __restrict__ f1, int ld1, R* __restrict__ f3,
+                                                               int ld3, int m0, int mcount) {
+  const int npair = (mcount + 1) / 2, x = blockIdx.x / npair, q = 2 * (blockIdx.x - x * npair);
+  const int ib = A.i0 + x * blockDim.x, i = ib + threadIdx.x;
+  prefetch_rows(f1, ld1, A.KL, ib, min((int)blockDim.x, A.i1 - ib), m0 + q, q + 1 < mcount);
+  if (i >= A.i1) return;
+  propags_pair_cur<R, VAR, RED, REFRD, CNT>(A, f1, ld1, f3, ld3, i, m0 + q, q + 1 < mcount);
 }
 
 // Batched form: every member of an ensemble (one coefficient family) in one
@@ -316,16 +514,19 @@ __global__ void __launch_bounds__(BS) propags_batch_kernel(const PropMember<R>* 
   __syncthreads();
   const int lb = (int)blockIdx.x - first[g], r = lb / sm.nbi;
   const int ib = sm.A.i0 + (lb - r * sm.nbi) * BS, i = ib + threadIdx.x;
-  if constexpr (!Site<R, VAR, RED, REFRD>::CUR) {
-    if (sm.pair) {
-      const int m = 2 * r;
-      const bool two = m + 1 < sm.A.ML;
-      prefetch_rows(sm.src, sm.ld, sm.A.KL, ib, min(BS, sm.A.i1 - ib), m, two);
-      if (i >= sm.A.i1) return;
+  if (sm.pair) {
+    const int m = 2 * r;
+    const bool two = m + 1 < sm.A.ML;
+    prefetch_rows(sm.src, sm.ld, sm.A.KL, ib, min(BS, sm.A.i1 - ib), m, two);
+    if (i >= sm.A.i1) return;
+    if constexpr (Site<R, VAR, RED, REFRD>::CUR) {
+      if (sm.A.counter == 1) propags_pair_cur<R, VAR, RED, REFRD, false>(sm.A, sm.src, sm.ld, sm.dst, sm.ld, i, m, two);
+      else propags_pair_cur<R, VAR, RED, REFRD, true>(sm.A, sm.src, sm.ld, sm.dst, sm.ld, i, m, two);
+    } else {
       if (sm.A.counter == 1) propags_pair<R, VAR, RED, REFRD, false>(sm.A, sm.src, sm.ld, sm.dst, sm.ld, i, m, two);
       else propags_pair<R, VAR, RED, REFRD, true>(sm.A, sm.src, sm.ld, sm.dst, sm.ld, i, m, two);
-      return;
     }
+    return;
   }
   if (i >= sm.A.i1) return;
   propags_point<R, VAR, RED, REFRD>(sm.A, sm.src, sm.ld, sm.dst, sm.ld, i, r);
@@ -444,9 +645,14 @@ cudaError_t dispatch(const PropArgs<R>& A, Args&&... args) {
 
 template <typename R, int V, bool RED, bool RD> struct PropLaunch {
   static cudaError_t run(const PropArgs<R>& A, const R* f1, int ld1, R* f3, int ld3, int m0, int mcount, cudaStream_t s) {
-    if constexpr (!var_current(V)) if (propags_pairs(A, std::max(ld1, ld3))) {
+    if (propags_pairs(A, std::max(ld1, ld3))) {
       const dim3 grid((A.i1 - A.i0 + 127) / 128, (mcount + 1) / 2);
-      if (A.counter == 1) propags_pair_kernel<R, V, RED, RD, false><<<grid, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
+      if constexpr (var_current(V)) {
+        // the current's refraction is not switched off by REFRD: one instance
+        const unsigned n = grid.x * grid.y;
+        if (A.counter == 1) propags_pair_cur_kernel<R, V, RED, false, false><<<n, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
+        else propags_pair_cur_kernel<R, V, RED, false, true><<<n, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
+      } else if (A.counter == 1) propags_pair_kernel<R, V, RED, RD, false><<<grid, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
       else propags_pair_kernel<R, V, RED, RD, true><<<grid, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
       return cudaGetLastError();
     }
