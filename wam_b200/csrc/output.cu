@@ -5,17 +5,23 @@
 //
 // A CTA of six warps integrates 32 sea points, lane = point.  The spectrum
 // FL3(IJ,K,M) has the sea point fastest, so a warp reads 128 contiguous bytes
-// of every bin.  The warps first take frequencies (the sums over directions),
-// then directions (the sums over frequencies), so that every sum is one
-// thread's loop in the reference's order with its loads in flight together; the
-// second reading comes from L2, where a CTA's 138 KB still lie.  The integrals
-// are then dealt out to the warps.  One thread per point, the direction sums in
-// shared memory, had 18 warps on an SM wait for one chain of loads each: 84k
-// points, 36x30, the parameters and the wind sea / swell split together 1275 us,
-// now 407 us (a reading of the spectrum from DRAM takes 56 us; each of the two
-// calls needs one).  The unit is compiled without FMA contraction, so the
-// results are those of the reference's separate operations; only ATAN2 (current
-// direction, mean direction) is the device library's.
+// of every bin.  The warps take frequencies for the sums over directions and
+// directions for the sums over frequencies, so that every sum is one thread's
+// loop in the reference's order; the integrals are then dealt out to the warps.
+// One thread per point, the direction sums in shared memory, had 18 warps on an
+// SM wait for one chain of loads each.  84k points, 36x30, the parameters and
+// the wind sea / swell split together: 1275 us then, 290 us now (reading the
+// spectrum once from DRAM takes 56 us; each of the two calls has to).
+//   - output_kernel (121 us) reads each bin once, six frequencies on their way
+//     to shared memory while six are summed; reading the spectrum twice, the
+//     second time along the frequencies, took 236 us, since eight CTAs on an SM
+//     hold more than L2 does.
+//   - swell_kernel (168 us) does read it twice: bound by issue (54 % of the
+//     slots), and with the staging rows in shared memory too few warps fit
+//     (248 us).
+// The unit is compiled without FMA contraction, so the results are those of the
+// reference's separate operations; only ATAN2 (current direction, mean
+// direction) is the device library's.
 //
 // Routines (wam_interface_module.f90): TOTAL_ENERGY_B :1342-1410, FEMEAN
 // :207-286, TM1_TM2_PERIODS_B :1152-1245, PEAK_PERIOD_B :741-813,
@@ -128,26 +134,43 @@ __global__ void __launch_bounds__(kOutWarps * 32) output_kernel(const __grid_con
   const R DEG = OutConst<R>::DEG;
   R* Tk = reinterpret_cast<R*>(smem_raw) + lane;  // [k * 32]: direction sums over frequency
   R* Tm = Tk + kl * 32;                           // [m * 32]: frequency spectrum (sum over directions)
-  R* DF = Tm + ml * 32 - lane;                    // DFIM
+  R* X = Tm + ml * 32;                            // twice six frequencies of the spectrum
+  R* DF = X + 2 * kOutWarps * kl * 32 - lane;     // DFIM
   for (int m = threadIdx.x; m < ml; m += kOutWarps * 32) DF[m] = a.DFIM[m];
   __syncthreads();
-  const R* f = a.fl3 + ij;
-  for (int m = w; m < ml; m += kOutWarps) {
-    const R* fm = f + (size_t)a.ld * kl * m;
-    R s = R(0);
+  // six frequencies on their way while six are summed
+  auto load = [&](int m0, int buf) {
+    if (m0 + w < ml) {
+      const R* fm = a.fl3 + ij + (size_t)a.ld * kl * (m0 + w);
+      unsigned x = (unsigned)__cvta_generic_to_shared(X + (buf * kOutWarps + w) * kl * 32);
+#pragma unroll 4
+      for (int k = 0; k < kl; ++k, fm += a.ld, x += 32 * sizeof(R))
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(x), "l"(fm), "n"(sizeof(R)) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  load(0, 0);
+  for (int m0 = 0, buf = 0; m0 < ml; m0 += kOutWarps, buf ^= 1) {
+    load(m0 + kOutWarps, buf ^ 1);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    const int nm = min(kOutWarps, ml - m0);
+    const R* x = X + buf * kOutWarps * kl * 32;
+    if (w < nm) {
+      R s = R(0);
 #pragma unroll 12
-    for (int k = 0; k < kl; ++k, fm += a.ld) s = s + __ldg(fm);
-    Tm[m * 32] = s;
+      for (int k = 0; k < kl; ++k) s = s + x[(w * kl + k) * 32];
+      Tm[(m0 + w) * 32] = s;
+    }
+    for (int k = w; k < kl; k += kOutWarps) {
+      R t = m0 == 0 ? R(0) : Tk[k * 32];
+#pragma unroll
+      for (int j = 0; j < kOutWarps; ++j)
+        if (j < nm) t = t + x[(j * kl + k) * 32] * DF[m0 + j];
+      Tk[k * 32] = t;
+    }
+    __syncthreads();
   }
-  for (int k = w; k < kl; k += kOutWarps) {
-    const R* fk = f + (size_t)a.ld * k;
-    const size_t step = (size_t)a.ld * kl;
-    R t = R(0);
-#pragma unroll 10
-    for (int m = 0; m < ml; ++m, fk += step) t = t + __ldg(fk) * DF[m];
-    Tk[k * 32] = t;
-  }
-  __syncthreads();
   R* out = a.block + ij;
   auto put = [&](int p, R v) { if (real) out[(size_t)a.block_ld * (p - 1)] = v; };
   if (w == 0) {
@@ -267,7 +290,7 @@ __global__ void __launch_bounds__(kOutWarps * 32) swell_kernel(const __grid_cons
   else direction_part(a, swell ? Tk1 : Tk4, put, p + 5);
 }
 
-template <typename R> size_t output_smem(int KL, int ML) { return (size_t)(32 * (KL + ML) + ML) * sizeof(R); }
+template <typename R> size_t output_smem(int KL, int ML) { return (size_t)(32 * ((1 + 2 * kOutWarps) * KL + ML) + ML) * sizeof(R); }
 template <typename R> size_t swell_smem(int KL, int ML) { return (size_t)(32 * (3 * KL + 2 * ML) + 2 * ML) * sizeof(R); }
 
 }  // namespace
@@ -275,12 +298,10 @@ template <typename R> size_t swell_smem(int KL, int ML) { return (size_t)(32 * (
 template <typename R> cudaError_t launch_swell(const OutArgs<R>& a, cudaStream_t s) {
   if (a.nsea == 0) return cudaSuccess;
   const size_t smem = swell_smem<R>(a.KL, a.ML);
-  static bool raised[2] = {false, false};
-  if (smem > 48 * 1024 && !raised[sizeof(R) == 8]) {
+  if (smem > 48 * 1024) {  // the limit belongs to the current device
     cudaError_t e = cudaFuncSetAttribute(swell_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)swell_smem<R>(MAX_KL, MAX_ML));
     if (e != cudaSuccess) return e;
-    raised[sizeof(R) == 8] = true;
   }
   swell_kernel<R><<<(a.nsea + 31) / 32, kOutWarps * 32, smem, s>>>(a);
   return cudaGetLastError();
@@ -421,12 +442,10 @@ template <typename R> cudaError_t launch_output(const OutArgs<R>& a, unsigned lo
     b.ustar_max = ustar_max;
   }
   const size_t smem = output_smem<R>(a.KL, a.ML);
-  static bool raised[2] = {false, false};
-  if (smem > 48 * 1024 && !raised[sizeof(R) == 8]) {
+  if (smem > 48 * 1024) {  // the limit belongs to the current device
     cudaError_t e = cudaFuncSetAttribute(output_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)output_smem<R>(MAX_KL, MAX_ML));
     if (e != cudaSuccess) return e;
-    raised[sizeof(R) == 8] = true;
   }
   output_kernel<R><<<(a.nsea + 31) / 32, kOutWarps * 32, smem, s>>>(b);
   return cudaGetLastError();
