@@ -1703,10 +1703,16 @@ int batch_impl_lists(wamgpu_batch* b, const std::vector<int>& Pin, std::vector<B
   return WAMGPU_OK;
 }
 
+template <typename R> int launch_impl_list(wamgpu_batch* b, const BatchList& L, cudaStream_t s) {
+  BCK(launch_implsch_batch<R>(impl_of<R>(b->members[L.family]).dt, L.mem.template as<ImplArgs<R>>(),
+                              L.first.template as<int>(), L.nmem, L.nblocks, L.P, L.smem, s), "batched IMPLSCH");
+  return WAMGPU_OK;
+}
 template <typename R> int launch_impl_lists(wamgpu_batch* b, const std::vector<BatchList>& Ls, cudaStream_t s) {
-  for (const BatchList& L : Ls)
-    BCK(launch_implsch_batch<R>(impl_of<R>(b->members[L.family]).dt, L.mem.template as<ImplArgs<R>>(),
-                                L.first.template as<int>(), L.nmem, L.nblocks, L.P, L.smem, s), "batched IMPLSCH");
+  for (const BatchList& L : Ls) {
+    const int rc = launch_impl_list<R>(b, L, s);
+    if (rc) return rc;
+  }
   return WAMGPU_OK;
 }
 
@@ -1764,14 +1770,49 @@ template <typename R> int batch_build(wamgpu_batch* b, cudaStream_t s) {
   return WAMGPU_OK;
 }
 
-template <typename R> int batch_launch(wamgpu_batch* b, cudaStream_t s) {
+// Side streams of one capture: they and their events end with it, the graph
+// keeps the branches.
+struct Branches {
+  std::vector<cudaStream_t> streams;
+  std::vector<cudaEvent_t> events;
+  cudaError_t add() {
+    cudaStream_t x = nullptr;
+    cudaEvent_t e = nullptr;
+    cudaError_t rc = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+    if (rc != cudaSuccess) return rc;
+    events.push_back(e);
+    if ((rc = cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking)) == cudaSuccess) streams.push_back(x);
+    return rc;
+  }
+  ~Branches() {
+    for (cudaStream_t x : streams) cudaStreamDestroy(x);
+    for (cudaEvent_t e : events) cudaEventDestroy(e);
+  }
+};
+
+// One pass of all members.  With branches (capture) every source-table class but
+// the first runs IMPLSCH on a branch of its own: a class is a few waves of tiles,
+// one per SM, whose last wave leaves most SMs idle, and the next class fills
+// them.  Eight members of 1k-47k points in four classes: 5.08 -> 4.94 ms a pass.
+template <typename R> int batch_launch(wamgpu_batch* b, cudaStream_t s, Branches* br = nullptr) {
   for (auto& step : b->sub)
     for (auto& L : step) {
       const PropArgs<R>& fam = impl_of<R>(b->members[L.family]).pa;
       BCK(launch_propags_batch<R>(fam, L.mem.template as<PropMember<R>>(), L.first.template as<int>(), L.nmem, L.nblocks,
                                   b->bs, s), "batched PROPAGS");
     }
-  return launch_impl_lists<R>(b, b->imp, s);
+  if (!br || b->imp.size() < 2) return launch_impl_lists<R>(b, b->imp, s);
+  BCK(cudaEventRecord(br->events[0], s), "fork");
+  for (size_t c = 1; c < b->imp.size(); ++c) {
+    BCK(cudaStreamWaitEvent(br->streams[c], br->events[0], 0), "fork");
+    const int rc = launch_impl_list<R>(b, b->imp[c], br->streams[c]);
+    if (rc) return rc;
+    BCK(cudaEventRecord(br->events[c], br->streams[c]), "join");
+  }
+  const int rc = launch_impl_list<R>(b, b->imp[0], s);
+  if (rc) return rc;
+  for (size_t c = 1; c < b->imp.size(); ++c) BCK(cudaStreamWaitEvent(s, br->events[c], 0), "join");
+  return WAMGPU_OK;
 }
 
 // Autotuner: times the first batched PROPAGS sub-step with 128- and 256-point
@@ -2282,8 +2323,10 @@ int wamgpu_batch_capture(wamgpu_batch* b, void* stream) {
     int rc = b->precision == 8 ? batch_build<double>(b, s) : batch_build<float>(b, s);
     if (rc) return rc;
   }
+  Branches br;
+  for (size_t c = 0; c < b->imp.size(); ++c) BCK(br.add(), "branch");
   BCK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "begin capture");
-  int rc = b->precision == 8 ? batch_launch<double>(b, s) : batch_launch<float>(b, s);
+  int rc = b->precision == 8 ? batch_launch<double>(b, s, &br) : batch_launch<float>(b, s, &br);
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamEndCapture(s, &g);
   if (rc) { if (g) cudaGraphDestroy(g); return rc; }
