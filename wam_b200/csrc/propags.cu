@@ -67,11 +67,13 @@ __global__ void __launch_bounds__(128) propags_kernel(const __grid_constant__ Pr
 //   - a land neighbour is read as the point itself and replaced by 0;
 //   - row offsets are 32-bit and run along;
 //   - CHECK_CFL's division by COUNTER runs as an exact scaled Markstein quotient.
-// 105 -> 67 thread instructions per bin (32 of them FP32) on the shallow
+// 105 -> 70 thread instructions per bin (32 of them FP32) on the shallow
 // spherical grid with depth refraction.  A sub-step of 756k points, 36x30, takes
-// 1.98 ms (3.3 TB/s of algorithmic traffic) against 2.69 before, with COUNTER = 2
+// 1.93 ms (3.4 TB/s of algorithmic traffic) against 2.69 before, with COUNTER = 2
 // on 159k points 36x35 0.67 against 1.39, deep on 47k points 24x25 0.074 against
-// 0.100.  Now bound by issue (71 % of the slots) and the latency of L2: three
+// 0.100.  The pairs of a block of points run next to each other (the blocks of a
+// pair next to each other instead: 1.98 ms).
+// Now bound by issue (78 % of the slots) and the latency of L2: three
 // directions in flight are the most that 64 registers hold (unrolled by 1, 2 or
 // 4 without the prefetch below: 4.1, 3.5 and 2.8 ms); the leaner deep stencil
 // takes six.
@@ -471,7 +473,8 @@ __device__ __forceinline__ void prefetch_rows(const R* __restrict__ f1, int ld1,
 template <typename R, int VAR, bool RED, bool REFRD, bool CNT>
 __global__ void __launch_bounds__(128) propags_pair_kernel(const __grid_constant__ PropArgs<R> A, const R* __restrict__ f1,
                                                            int ld1, R* __restrict__ f3, int ld3, int m0, int mcount) {
-  const int ib = A.i0 + blockIdx.x * blockDim.x, i = ib + threadIdx.x, q = 2 * blockIdx.y;
+  const int npair = (mcount + 1) / 2, x = blockIdx.x / npair, q = 2 * (blockIdx.x - x * npair);
+  const int ib = A.i0 + x * blockDim.x, i = ib + threadIdx.x;
   prefetch_rows(f1, ld1, A.KL, ib, min((int)blockDim.x, A.i1 - ib), m0 + q, q + 1 < mcount);
   if (i >= A.i1) return;
   propags_pair<R, VAR, RED, REFRD, CNT>(A, f1, ld1, f3, ld3, i, m0 + q, q + 1 < mcount);
@@ -646,14 +649,13 @@ cudaError_t dispatch(const PropArgs<R>& A, Args&&... args) {
 template <typename R, int V, bool RED, bool RD> struct PropLaunch {
   static cudaError_t run(const PropArgs<R>& A, const R* f1, int ld1, R* f3, int ld3, int m0, int mcount, cudaStream_t s) {
     if (propags_pairs(A, std::max(ld1, ld3))) {
-      const dim3 grid((A.i1 - A.i0 + 127) / 128, (mcount + 1) / 2);
+      const unsigned n = (unsigned)((A.i1 - A.i0 + 127) / 128) * ((mcount + 1) / 2);
       if constexpr (var_current(V)) {
         // the current's refraction is not switched off by REFRD: one instance
-        const unsigned n = grid.x * grid.y;
         if (A.counter == 1) propags_pair_cur_kernel<R, V, RED, false, false><<<n, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
         else propags_pair_cur_kernel<R, V, RED, false, true><<<n, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
-      } else if (A.counter == 1) propags_pair_kernel<R, V, RED, RD, false><<<grid, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
-      else propags_pair_kernel<R, V, RED, RD, true><<<grid, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
+      } else if (A.counter == 1) propags_pair_kernel<R, V, RED, RD, false><<<n, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
+      else propags_pair_kernel<R, V, RED, RD, true><<<n, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
       return cudaGetLastError();
     }
     dim3 grid((A.i1 - A.i0 + 127) / 128, mcount);
