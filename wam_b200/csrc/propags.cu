@@ -646,10 +646,15 @@ cudaError_t dispatch(const PropArgs<R>& A, Args&&... args) {
   return cudaErrorInvalidValue;
 }
 
+// A launch of no more CTAs than this lasts as long as one thread's walk along the
+// directions, which is shorter with one frequency unless there are currents (135
+// points, 36x30, shallow with depth refraction, the call with its copy: 18.6 us
+// against 22.6; with currents 35.0 against 28.8).
+constexpr unsigned PAIR_MIN_CTAS = 32;
 template <typename R, int V, bool RED, bool RD> struct PropLaunch {
   static cudaError_t run(const PropArgs<R>& A, const R* f1, int ld1, R* f3, int ld3, int m0, int mcount, cudaStream_t s) {
-    if (propags_pairs(A, std::max(ld1, ld3))) {
-      const unsigned n = (unsigned)((A.i1 - A.i0 + 127) / 128) * ((mcount + 1) / 2);
+    const unsigned n = (unsigned)((A.i1 - A.i0 + 127) / 128) * ((mcount + 1) / 2);
+    if (propags_pairs(A, std::max(ld1, ld3)) && (var_current(V) || n > PAIR_MIN_CTAS)) {
       if constexpr (var_current(V)) {
         // the current's refraction is not switched off by REFRD: one instance
         if (A.counter == 1) propags_pair_cur_kernel<R, V, RED, false, false><<<n, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
