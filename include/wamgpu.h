@@ -221,6 +221,10 @@ WAMGPU_API int wamgpu_propags_substep_dev(wamgpu_ctx* ctx, const void* src, void
 WAMGPU_API int wamgpu_propags_substep_range_dev(wamgpu_ctx* ctx, const void* src, void* dst, int ld, int i0, int i1,
                                                 void* stream);
 WAMGPU_API int wamgpu_get_halo_width(const wamgpu_ctx* ctx);
+/* Sea points per CTA of the context's IMPLSCH (test diagnostics): 32 where it
+ * runs on tiles of points, fewer where one warp integrates one point.  Both
+ * give the same bits.  A negative code without a grid. */
+WAMGPU_API int wamgpu_get_implsch_points(const wamgpu_ctx* ctx);
 
 /* Batched ensembles.  No single counterpart in the reference, where each
  * member is a separate WAMODEL run calling PROPAGS (propagation:635-829) and

@@ -75,6 +75,7 @@ SIGNATURES = {
     "wamgpu_propags_substep_dev": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p]),
     "wamgpu_propags_substep_range_dev": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "wamgpu_get_halo_width": (c_int, [c_void_p]),
+    "wamgpu_get_implsch_points": (c_int, [c_void_p]),
     "wamgpu_batch_create": (c_int, [ctypes.POINTER(c_void_p), c_int, ctypes.POINTER(c_void_p)]),
     "wamgpu_batch_destroy": (c_int, [c_void_p]),
     "wamgpu_batch_last_error": (c_char_p, [c_void_p]),

@@ -180,9 +180,9 @@ template <typename R> bool tile_geometry(const TableSet<R>& t) {
 // longer hold at once: up to there that kernel takes one wave, and a point of
 // its own per warp is done sooner than a tile (135 points, ST4, KL=24: 151 us
 // against 182; 1485 points, ST6, KL=36: 84 against 121), beyond it takes two and
-// more (1800 points: 302 against 182, 149 against 120).  The rule looks at the
-// context's whole grid, so chunks, owned ranges and ensemble members of one
-// context all run on the same kernel and agree bit for bit.
+// more (1800 points: 302 against 182, 149 against 120).  Both forms give the same
+// bits (implsch.cuh), so a grid's bands, which may fall on the other side,
+// reproduce it.
 template <typename R> int cta_points(const wamgpu_ctx* ctx, const DevTables<R>& d) {
   return d.tile.smem && ctx->nsea > ctx->wave ? 32 : ctx->P;
 }
@@ -2373,6 +2373,12 @@ int wamgpu_propags_substep_range_dev(wamgpu_ctx* ctx, const void* src, void* dst
 int wamgpu_get_halo_width(const wamgpu_ctx* ctx) {
   if (!ctx || !ctx->have_grid) return WAMGPU_E_STATE;
   return ctx->halo;
+}
+
+int wamgpu_get_implsch_points(const wamgpu_ctx* ctx) {
+  if (!ctx || !ctx->impl || !ctx->have_grid) return WAMGPU_E_STATE;
+  wamgpu_ctx* c = const_cast<wamgpu_ctx*>(ctx);
+  return c->cfg.precision == 8 ? cta_points(c, impl_of<double>(c).dt) : cta_points(c, impl_of<float>(c).dt);
 }
 
 int wamgpu_propags_substep_dev(wamgpu_ctx* ctx, const void* src, void* dst, int ld, void* stream) {

@@ -47,6 +47,9 @@ __device__ __forceinline__ float radd(float a, float b) { return __fadd_rn(a, b)
 __device__ __forceinline__ double radd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ float rsub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ double rsub(double a, double b) { return __dsub_rn(a, b); }
+// a * b + c rounded once.
+__device__ __forceinline__ float rfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double rfma(double a, double b, double c) { return __fma_rn(a, b, c); }
 // Two single-precision operations per instruction (fma.rn.f32x2 and the like):
 // each half rounds as the scalar operation does, but the compiler fuses an add2
 // of a mul2 into one rounding, .rn or not (seen on sm_100a, CUDA 12.9): sums of

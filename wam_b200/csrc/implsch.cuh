@@ -28,6 +28,15 @@
 // Two reference computations whose results IMPLSCH never reads are not
 // evaluated: TAU_WAVE_ATMOS (TAUNW of SINPUT_ST6) and, for ST6 without
 // LCFLX, STRESSO (its TAUW is a dummy and PHIAW only feeds the flux module).
+//
+// Rounding.  The single-precision step has a second form, on tiles of points
+// (implsch_tile.cuh), and which of the two runs depends on the size of a
+// context's grid.  They give the same bits: every sum or difference that a
+// product could be contracted into is written with its rounding (rfma rounds
+// once; radd and rsub, which are never contracted, after the product), in the
+// same order in both, so that nothing is left to the compiler's choice.  A bit matters: the integer decisions of
+// the step (wind-sea mask, cut-off indices, LFACTOR's iterations) would
+// otherwise fall apart where a value lies on their thresholds.
 #pragma once
 #include <cstdint>
 #include <cfloat>
@@ -116,6 +125,11 @@ template <typename R> __host__ __device__ inline size_t tables_bytes(const Small
   size_t b = (size_t)L.nreal * sizeof(R) + (size_t)L.nint * sizeof(int);
   return (b + 15) & ~size_t(15);
 }
+
+// LOG10(x) - 0.3 of SINPUT_ARD's swell friction table, a function of its own so
+// that the library function's last operation meets the difference in the same
+// code wherever it is used.
+template <typename R> __device__ __noinline__ R swell_log(R x) { return dlog10(x) - R(0.3); }
 
 // Per-point outputs of IMPLSCH beyond the spectrum.
 template <typename R> struct PointState {
@@ -267,21 +281,22 @@ template <typename R> struct Src {
   __device__ void airsea(R TAUW, R& USTAR, R& Z0) const {
     const R EPS1 = R(0.00001);
     R xlogxl = dlog(P_::XNLEV), alphaog = T.ALPHA / P_::G, xkutop = P_::XKAPPA * U10;
-    R ustold = U10 * dsqrt(R(8.0E-4) + R(8.0E-5) * U10);
-    R tauold = dmax(ustold * ustold, TAUW + EPS1);
+    R ustold = U10 * dsqrt(rfma(R(8.0E-5), U10, R(8.0E-4)));
+    R tauold = dmax(ustold * ustold, radd(TAUW, EPS1));
     USTAR = dsqrt(tauold);
     R ustm1 = R(1.0) / dmax(USTAR, R(1.0E-6));
     R z0ch = 0;
     for (int it = 0; it < 15; ++it) {
       R x = TAUW / tauold;
-      z0ch = alphaog * tauold / dsqrt(dmax(R(1.0) - x, EPS1));
-      R z0vis = P_::RNUAIRM * ustm1, z0tot = z0ch + z0vis;
-      R xologz0 = R(1.0) / (xlogxl - dlog(z0tot));
-      R f = USTAR - xkutop * xologz0;
-      R zz = ustm1 * (z0ch * (R(2.0) - R(3.0) * x) / (R(1.0) - x) - z0vis) / z0tot;
-      R delf = R(1.0) - xkutop * (xologz0 * xologz0) * zz;
-      USTAR = USTAR - f / delf;
-      R taunew = dmax(USTAR * USTAR, TAUW + EPS1);
+      z0ch = alphaog * tauold / dsqrt(dmax(rsub(R(1.0), x), EPS1));
+      R z0tot = rfma(P_::RNUAIRM, ustm1, z0ch);
+      R xologz0 = R(1.0) / rsub(xlogxl, dlog(z0tot));
+      R f = rfma(-xkutop, xologz0, USTAR);
+      R zc = z0ch * rfma(R(-3.0), x, R(2.0)) / rsub(R(1.0), x);
+      R zz = ustm1 * rfma(-P_::RNUAIRM, ustm1, zc) / z0tot;
+      R delf = rfma(-(xkutop * (xologz0 * xologz0)), zz, R(1.0));
+      USTAR = rsub(USTAR, f / delf);
+      R taunew = dmax(USTAR * USTAR, radd(TAUW, EPS1));
       USTAR = dsqrt(taunew);
       if (taunew == tauold) break;
       ustm1 = R(1.0) / dmax(USTAR, R(1.0E-6));
@@ -303,12 +318,12 @@ template <typename R> struct Src {
 
   __device__ R wsigstar(R ustar, R z0) const {
     const R C1 = R(1.03E-3), C2 = R(0.04E-3), P1 = R(1.48), P2 = R(-0.21);
-    R u = ustar * (R(1.0) / P_::XKAPPA) * (dlog(R(10.0)) - dlog(z0));
+    R u = ustar * (R(1.0) / P_::XKAPPA) * rsub(dlog(R(10.0)), dlog(z0));
     u = dmax(u, R(1.0));
     R um1 = R(1.0) / u, c2u = C2 * dpow(u, P1), up2 = dpow(u, P2);
-    R cdv = (C1 + c2u) * up2;
-    R dcd = (P2 * C1 + (P1 + P2) * c2u) * up2 * um1;
-    R sconv = R(1.0) + R(0.5) * u / cdv * dcd;
+    R cdv = radd(C1, c2u) * up2;
+    R dcd = rfma(P1 + P2, c2u, P2 * C1) * up2 * um1;
+    R sconv = rfma(R(0.5) * u / cdv, dcd, R(1.0));
     return dmin(R(0.1), sconv * um1 * dpow(R(0.5) * P_::XKAPPA * (WSTAR * WSTAR * WSTAR), R(1.0) / R(3.0)));
   }
 
@@ -335,22 +350,23 @@ template <typename R> struct Src {
       R t = 0;
       for (int k = 0; k < kl; ++k) t = t + w.F[k + ld * m];
       R sig = P_::ZPI * S.FR[m];
-      uo = uo + S.DFIM[m] * (sig * sig) * t;
-      ao = ao + S.DFIM[m] * t;
+      uo = rfma(S.DFIM[m] * (sig * sig), t, uo);
+      ao = rfma(S.DFIM[m], t, ao);
     }
     R tiny = sizeof(R) == 4 ? R(FLT_MIN) : R(DBL_MIN);
-    R uorbt = R(2.0) * dsqrt(tiny + warp_sum(uo));
-    R aorb = R(2.0) * dsqrt(tiny + warp_sum(ao));
-    R re = (R(4.0) / nu) * uorbt * aorb;
+    R uorbt = R(2.0) * dsqrt(radd(tiny, warp_sum(uo)));
+    R aorb = R(2.0) * dsqrt(radd(tiny, warp_sum(ao)));
+    R re = rfma((R(4.0) / nu) * uorbt, aorb, -SWELLF4);
     R z0noz = dmax(P_::RNUAIRM / dmax(USTAR, R(0.0001)), R(0.04) * dmin(R(0.0005), Z0));
-    R xi = (dlog10(dmax(aorb / z0noz, R(3.0))) - R(0.3)) * delabm1;
+    R xi = swell_log(dmax(aorb / z0noz, R(3.0))) * delabm1;
     int ind = min(199, max(1, (int)xi));  // xi >= 4.6 for finite input; clamp keeps NaN input in bounds
-    R deli1 = dmin(R(1.0), xi - R(ind));
-    R fww = S.SWELLFT[ind - 1] * (R(1.0) - deli1) + S.SWELLFT[ind] * deli1;
+    R deli1 = dmin(R(1.0), rsub(xi, R(ind)));
+    R fww = rfma(S.SWELLFT[ind], deli1, S.SWELLFT[ind - 1] * rsub(R(1.0), deli1));
     R temp2 = fww * uorbt;
-    R smooth = R(0.5) * dtanh((re - SWELLF4) / SWELLF7);
-    R pturb = R(0.5) + smooth, pvisc = R(0.5) - smooth;
-    R usg[2] = {(USTAR * (R(1.0) + sig_n)) * (USTAR * (R(1.0) + sig_n)), (USTAR * (R(1.0) - sig_n)) * (USTAR * (R(1.0) - sig_n))};
+    R smooth = R(0.5) * dtanh(re / SWELLF7);
+    R pturb = radd(R(0.5), smooth), pvisc = rsub(R(0.5), smooth);
+    R ug[2] = {USTAR * radd(R(1.0), sig_n), USTAR * rsub(R(1.0), sig_n)};
+    R usg[2] = {ug[0] * ug[0], ug[1] * ug[1]};
     R su = dsin(UDIR), cu = dcos(UDIR);
     R taux[2] = {usg[0] * su, usg[1] * su}, tauy[2] = {usg[0] * cu, usg[1] * cu};
     R xst[2] = {0, 0}, yst[2] = {0, 0};
@@ -363,21 +379,21 @@ template <typename R> struct Src {
       else { cm = sig / P_::G; xk = sig2 / P_::G; }
       R ustp[2], usdirp[2], cu_[2], su_[2], ucn[2], ucnz[2];
       for (int g = 0; g < 2; ++g) {
-        R tpx = taux[g] - shelter * xst[g], tpy = tauy[g] - shelter * yst[g];
+        R tpx = rfma(-shelter, xst[g], taux[g]), tpy = rfma(-shelter, yst[g], tauy[g]);
+        const R qq = rfma(tpx, tpx, tpy * tpy);
         if constexpr (TAB) {
-          const R qq = tpx * tpx + tpy * tpy;
           ustp[g] = dsqrt(dsqrt(qq));
           const R rn = qq > R(0) ? R(1) / dsqrt(qq) : R(0);
           cu_[g] = qq > R(0) ? tpy * rn : R(1);
           su_[g] = tpx * rn;
           usdirp[g] = R(0);
         } else {
-          ustp[g] = dpow(tpx * tpx + tpy * tpy, R(0.25));
+          ustp[g] = dpow(qq, R(0.25));
           usdirp[g] = datan2(tpx, tpy);
           cu_[g] = su_[g] = R(0);
         }
         ucn[g] = ustp[g] * cm;
-        ucnz[g] = P_::XKAPPA / (ucn[g] + T.ZALP);
+        ucnz[g] = P_::XKAPPA / radd(ustp[g] * cm, T.ZALP);
       }
       R constf = rogoroair * cm * S.DFIM[m];
       R zcn = dlog(xk * Z0);
@@ -392,29 +408,29 @@ template <typename R> struct Src {
         uint8_t ll = 0;
         for (int g = 0; g < 2; ++g) {
           R c;
-          if constexpr (TAB) c = S.COSTH[k] * cu_[g] + S.SINTH[k] * su_[g];
-          else c = dcos(S.TH[k] - usdirp[g]);
+          if constexpr (TAB) c = rfma(S.COSTH[k], cu_[g], S.SINTH[k] * su_[g]);
+          else c = dcos(rsub(S.TH[k], usdirp[g]));
           R ufac = 0;
           if (c > R(0.01)) {
-            R x = c * ucn[g], zlog = zcn + (TAB ? ucnz[g] * (R(1) / c) : ucnz[g] / c);
+            R x = c * ucn[g], zlog = TAB ? rfma(ucnz[g], R(1) / c, zcn) : radd(zcn, ucnz[g] / c);
             if (zlog < R(0.0)) { R z2x = zlog * zlog * x; ufac = dexp(zlog) * z2x * z2x; ll = 1; }
           }
-          R dstab = dstab1 + pturb * (tmp1 * (temp2 + (FU + FUD * c) * ustp[g]));
+          R dstab = rfma(pturb, tmp1 * rfma(rfma(FUD, c, FU), ustp[g], temp2), dstab1);
           slp[g] = cnsn * ufac;
-          flp[g] = slp[g] + dstab;
+          flp[g] = radd(slp[g], dstab);
           slp[g] = slp[g] * f;
-          px[g] = px[g] + slp[g] * (constf * S.SINTH[k]);
-          py[g] = py[g] + slp[g] * (constf * S.COSTH[k]);
+          px[g] = rfma(slp[g], constf * S.SINTH[k], px[g]);
+          py[g] = rfma(slp[g], constf * S.COSTH[k], py[g]);
         }
         int b = k + ld * m;
-        R spos = R(0.5) * (slp[0] + slp[1]);  // >= 0
+        R spos = R(0.5) * radd(slp[0], slp[1]);  // >= 0
         if (w.SP) w.SP[b] = spos;
-        st = st + spos; sx = sx + spos * S.SINTH[k]; sy = sy + spos * S.COSTH[k];
-        R fl = R(0.5) * (flp[0] + flp[1]);
+        st = radd(st, spos); sx = rfma(spos, S.SINTH[k], sx); sy = rfma(spos, S.COSTH[k], sy);
+        R fl = R(0.5) * radd(flp[0], flp[1]);
         w.SF[b] = r2(fl * f, fl);
         w.LL[b] = ll;
       }
-      for (int g = 0; g < 2; ++g) { xst[g] = xst[g] + warp_sum(px[g]); yst[g] = yst[g] + warp_sum(py[g]); }
+      for (int g = 0; g < 2; ++g) { xst[g] = radd(xst[g], warp_sum(px[g])); yst[g] = radd(yst[g], warp_sum(py[g])); }
       st = warp_sum(st); sx = warp_sum(sx); sy = warp_sum(sy);
       if (lane == 0) { ST[m] = st; SX[m] = sx; SY[m] = sy; }
     }
@@ -429,17 +445,17 @@ template <typename R> struct Src {
     R omegacc = dmax(omegac, T.X0TAUHF * P_::G / ustar);
     R sqrtz0og = dsqrt(z0 * gm1), sqrtgz0 = R(1.0) / sqrtz0og;
     R zinf = dlog(omegacc * sqrtz0og);
-    R delz = dmax((R(0.0) - zinf) / R(18), R(0.0));
+    R delz = dmax(-zinf / R(18), R(0.0));
     tauhf = 0; phihf = 0;
     for (int j = 0; j < 19; ++j) {
-      R y = dexp(zinf + R(j) * delz);
+      R y = dexp(rfma(R(j), delz, zinf));
       R cm1 = y * sqrtgz0 * gm1;
-      R zlog = dmin(xloggz0 + R(2.0) * dlog(cm1) + P_::XKAPPA / (ust * cm1 + T.ZALP), R(0.0));
+      R zlog = dmin(radd(rfma(R(2.0), dlog(cm1), xloggz0), P_::XKAPPA / rfma(ust, cm1, T.ZALP)), R(0.0));
       R z2 = zlog * zlog;
       R fnc2 = dexp(zlog) * (z2 * z2) * tauw * S.WTAUHF[j] * delz;
       ust = dsqrt(tauw);
-      tauhf = tauhf + fnc2;
-      phihf = phihf + fnc2 / y;
+      tauhf = radd(tauhf, fnc2);
+      phihf = radd(phihf, fnc2 / y);
     }
     phihf = sqrtz0og * phihf;
   }
@@ -452,21 +468,20 @@ template <typename R> struct Src {
     const R cst = T.DELTH * ((P_::ZPI * P_::ZPI) * (P_::ZPI * P_::ZPI)) * gm1;
     R t1 = 0, t2 = 0;
     for (int k = lane; k < kl; k += 32) {
-      R cw = dmax(dcos(S.TH[k] - UDIR), R(0.));
+      R cw = dmax(dcos(rsub(S.TH[k], UDIR)), R(0.));
       R f = w.F[k + ld * (mij - 1)];
-      t2 = t2 + f * (cw * cw);
-      t1 = t1 + f * (cw * cw * cw);
+      t2 = rfma(f, cw * cw, t2);
+      t1 = rfma(f, cw * cw * cw, t1);
     }
     pphi = warp_sum(pphi); px = warp_sum(px); py = warp_sum(py); t1 = warp_sum(t1); t2 = warp_sum(t2);
     R tau1, phi1;
     tau_phi_hf(mij, USTAR, Z0, tau1, phi1);
     R tauhf = cst * S.FR5[mij - 1] * gm1 * t1 * tau1;
-    R phihf = P_::ROAIR * cst * S.FR5[mij - 1] * t2 * phi1;
-    PHIAW = pphi + phihf;
-    R xs = px / P_::ROAIR + tauhf * dsin(UDIR);
-    R ys = py / P_::ROAIR + tauhf * dcos(UDIR);
-    R tw = dsqrt(xs * xs + ys * ys);
-    tw = dmin(tw, USTAR * USTAR - R(0.00001));
+    PHIAW = rfma(P_::ROAIR * cst * S.FR5[mij - 1] * t2, phi1, pphi);
+    R xs = rfma(tauhf, dsin(UDIR), px / P_::ROAIR);
+    R ys = rfma(tauhf, dcos(UDIR), py / P_::ROAIR);
+    R tw = dsqrt(rfma(xs, xs, ys * ys));
+    tw = dmin(tw, rsub(USTAR * USTAR, R(0.00001)));
     TAUW = dmax(tw, R(0.));
   }
   __device__ R rhowgdfth(int m, int mij) const {
@@ -482,7 +497,7 @@ template <typename R> struct Src {
     R pphi = 0, px = 0, py = 0;
     for (int m = lane; m < mij; m += 32) {
       R rw = rhowgdfth(m, mij), cmr = cmw(m) * rw;
-      pphi = pphi + ST[m] * rw; px = px + SX[m] * cmr; py = py + SY[m] * cmr;
+      pphi = rfma(ST[m], rw, pphi); px = rfma(SX[m], cmr, px); py = rfma(SY[m], cmr, py);
     }
     stresso_finish(USTAR, Z0, mij, pphi, px, py, TAUW, PHIAW);
   }
@@ -561,7 +576,7 @@ template <typename R> struct Src {
     const int kl = KL(), nw = 2 * T.NSDSNTH + 1;
     const R* fm = w.F + w.ld * m;
     R acc = 0;
-    for (int j = 0; j < nw; ++j) acc = acc + S.SATW[k + kl * j] * fm[S.INDSAT[k + kl * j] - 1];
+    for (int j = 0; j < nw; ++j) acc = rfma(S.SATW[k + kl * j], fm[S.INDSAT[k + kl * j] - 1], acc);
     return acc;
   }
   __device__ void sdissip_ard() const {
@@ -570,12 +585,12 @@ template <typename R> struct Src {
     const int nx = kl > 32 ? kl - 32 : 0, gsz = nx > 0 ? 32 / nx : ml;
     const int lg = nx > 0 ? lane / nx : 0, lx = nx > 0 ? lane - lg * nx : 0;
     auto whitecap = [&](int k, int m, R bth, R temp1, R ssdsc2_sig) {
-      R dd = dmax(R(0.), bth * tmp03 - R(1.0));
-      R d = ssdsc2_sig * (temp1 + c6m1 * (dd * dd));
+      R dd = dmax(R(0.), rfma(bth, tmp03, R(-1.0)));
+      R d = ssdsc2_sig * rfma(c6m1, dd * dd, temp1);
       int b = k + ld * m;
       R2 v = w.SF[b];
-      v.x = v.x + d * w.F[b];
-      v.y = v.y + d;
+      v.x = rfma(d, w.F[b], v.x);
+      v.y = radd(v.y, d);
       w.SF[b] = v;
     };
     for (int m0 = 0; m0 < ml; m0 += gsz) {
@@ -590,7 +605,7 @@ template <typename R> struct Src {
         if (lane < kl) { bth = sat_window(lane, m) * facsat; bmax = dmax(bmax, bth); }
         if (lact && lg == g) bmax = dmax(bmax, bthx);
         bmax = warp_max(bmax);
-        R d0 = dmax(R(0.), bmax * tmp03 - R(1.0));
+        R d0 = dmax(R(0.), rfma(bmax, tmp03, R(-1.0)));
         R temp1 = c6 * (d0 * d0);
         if (lg == g) temp1x = temp1;
         if (lane < kl) whitecap(lane, m, bth, temp1, R(-2.2E-5) * sig);
@@ -662,7 +677,7 @@ template <typename R> struct Src {
     R enhfr = R(1);
     if (T.shallow && T.isnonlin == 0) {
       enhfr = dmax(R(0.75) * DEPTH * AKMEAN, R(.5));
-      enhfr = R(1.) + (R(5.5) / enhfr) * (R(1.) - R(.833) * enhfr) * dexp(R(-1.25) * enhfr);
+      enhfr = rfma((R(5.5) / enhfr) * rfma(R(-.833), enhfr, R(1.)), dexp(R(-1.25) * enhfr), R(1.));
     }
     R2* SF = w.SF; const R* F = w.F;
     R2* XM = reinterpret_cast<R2*>(w.T);  // [kh*kl + k] = {AD, DELAM}
@@ -680,21 +695,20 @@ template <typename R> struct Src {
     auto interact = [&](const DiaMc& d, int k, R2* xm, R2* xp, int skh, R& adc, R& delc) {
       const Quad<R> c0 = ld4(d.rc), c1 = ld4(d.rc + 4);  // slots of RNLCOEF 0-4, 13-15
       const R g1 = c0.b, g2 = c0.c, g3 = c0.d, g4 = c1.a, g5 = c1.b, g6 = c1.c, g7 = c1.d, g8 = d.rc[8];
-      const R fij = F[k + d.rIC] * d.ftail;
+      const R fij = F[k + d.rIC] * d.ftail, fcen = d.ftemp * fij;
       adc = R(0); delc = R(0);
       for (int kh = 0; kh < 2; ++kh) {
         const int a1 = rot(k, o1[kh]), a11 = rot(k, o11[kh]), a2 = rot(k, o2[kh]), a21 = rot(k, o21[kh]);
-        R sap = g1 * F[a1 + d.rIP] + g2 * F[a11 + d.rIP] + g3 * F[a1 + d.rIP1] + g4 * F[a11 + d.rIP1];
-        R sam = g5 * F[a2 + d.rIM] + g6 * F[a21 + d.rIM] + g7 * F[a2 + d.rIM1] + g8 * F[a21 + d.rIM1];
-        R fad1 = fij * (sap + sam);
-        R fad2 = fad1 - R(2.) * sap * sam;
-        fad1 = fad1 + fad2;
-        R fcen = d.ftemp * fij;
+        const R sap = rfma(g4, F[a11 + d.rIP1], rfma(g3, F[a1 + d.rIP1], rfma(g1, F[a1 + d.rIP], g2 * F[a11 + d.rIP])));
+        const R sam = rfma(g8, F[a21 + d.rIM1], rfma(g7, F[a2 + d.rIM1], rfma(g5, F[a2 + d.rIM], g6 * F[a21 + d.rIM])));
+        R fad1 = fij * radd(sap, sam);
+        const R fad2 = rfma(R(-2.) * sap, sam, fad1);
+        fad1 = radd(fad1, fad2);
         const R ad = fad2 * fcen;
-        adc = adc + ad;
-        delc = delc + fad1 * d.ftemp;
-        xm[skh * kh] = r2(ad, (fij - R(2.) * sap) * T.DAL2 * fcen);
-        xp[skh * kh] = r2(ad, (fij - R(2.) * sam) * T.DAL1 * fcen);
+        adc = radd(adc, ad);
+        delc = rfma(fad1, d.ftemp, delc);
+        xm[skh * kh] = r2(ad, rfma(R(-2.), sap, fij) * T.DAL2 * fcen);
+        xp[skh * kh] = r2(ad, rfma(R(-2.), sam, fij) * T.DAL1 * fcen);
       }
     };
     // the target-row updates of column j from the KH-summed gathers
@@ -702,7 +716,8 @@ template <typename R> struct Src {
     // four weights (RNLCOEF slots 12 MM, 16 MM1, 20 MP, 24 MP1)
     auto upd = [&](const DiaMc& d, int slot, R2& v, R a, R dl, R b, R dm) {
       const Quad<R> c = ld4(d.rc + slot);
-      v.x = v.x + (a * c.a + b * c.b); v.y = v.y + (dl * c.c + dm * c.d);
+      v.x = radd(v.x, rfma(a, c.a, b * c.b));
+      v.y = radd(v.y, rfma(dl, c.c, dm * c.d));
     };
 
     const int kmain = kl < 32 ? kl : 32;          // directions of the per-MC pass (lane = k)
@@ -745,9 +760,9 @@ template <typename R> struct Src {
           const R2 p1a = XP[rot(j, kl - o1[0])], p1b = XP[kl + rot(j, kl - o1[1])];
           const R2 p11a = XP[rot(j, kl - o11[0])], p11b = XP[kl + rot(j, kl - o11[1])];
           R2 vC = SF[j + d.rMC], vM = SF[j + d.rMM], vM1 = SF[j + d.rMM1], vP = SF[j + d.rMP], vP1 = SF[j + d.rMP1];
-          const R a2 = m2a.x + m2b.x, d2 = m2a.y + m2b.y, a21 = m21a.x + m21b.x, d21 = m21a.y + m21b.y;
-          const R a1 = p1a.x + p1b.x, d1 = p1a.y + p1b.y, a11 = p11a.x + p11b.x, d11 = p11a.y + p11b.y;
-          if (d.wMC) { vC.x = vC.x - R(2.) * adc; vC.y = vC.y - R(2.) * delc; SF[j + d.rMC] = vC; }
+          const R a2 = radd(m2a.x, m2b.x), d2 = radd(m2a.y, m2b.y), a21 = radd(m21a.x, m21b.x), d21 = radd(m21a.y, m21b.y);
+          const R a1 = radd(p1a.x, p1b.x), d1 = radd(p1a.y, p1b.y), a11 = radd(p11a.x, p11b.x), d11 = radd(p11a.y, p11b.y);
+          if (d.wMC) { vC.x = rfma(R(-2.), adc, vC.x); vC.y = rfma(R(-2.), delc, vC.y); SF[j + d.rMC] = vC; }
           if (d.wMM) { upd(d, 12, vM, a2, d2, a21, d21); SF[j + d.rMM] = vM; }
           if (d.wMM1) { upd(d, 16, vM1, a2, d2, a21, d21); SF[j + d.rMM1] = vM1; }
           if (d.wMP) { upd(d, 20, vP, a1, d1, a11, d11); SF[j + d.rMP] = vP; }
@@ -775,7 +790,7 @@ template <typename R> struct Src {
           const R2* xs = XB + 4 * nx * lb + lx;
           s2 = xs[0]; s21 = xs[nx]; s1 = xs[2 * nx]; s11 = xs[3 * nx];
         }
-        if (lact && d.wMC) { R2 v = SF[j + d.rMC]; v.x = v.x - R(2.) * ladc; v.y = v.y - R(2.) * ldelc; SF[j + d.rMC] = v; }
+        if (lact && d.wMC) { R2 v = SF[j + d.rMC]; v.x = rfma(R(-2.), ladc, v.x); v.y = rfma(R(-2.), ldelc, v.y); SF[j + d.rMC] = v; }
         __syncwarp();
         if (lact && d.wMM) { R2 v = SF[j + d.rMM]; upd(d, 12, v, s2.x, s2.y, s21.x, s21.y); SF[j + d.rMM] = v; }
         __syncwarp();
@@ -863,7 +878,7 @@ template <typename R> struct Src {
         R w1 = dmax(R(0.), proj); w1 = w1 * w1;
         R w2 = dmin(R(0.), proj); w2 = w2 * w2;
         const bool up = proj > R(0.);
-        const R g = R(2.8) - (R(1.) + dtanh(rsub(rmul(R(10.) * sqb, up ? w1 : w2), R(11.))));
+        const R g = rsub(R(2.8), radd(R(1.), dtanh(rsub(rmul(R(10.) * sqb, up ? w1 : w2), R(11.)))));
         const R d1 = up ? raw * sig * g * sqb * w1 : R(0.);
         const R d2 = up ? R(0.) : raw * sig * R(0.09) * g * sqb * w2;
         sfm[k] = r2(d1, d2);
@@ -1076,7 +1091,7 @@ template <typename R> struct Src {
         const R2 v = w.SF[p];
         R d = v.x;
         if (reduce) d = d * lfm;
-        R dtot = d - v.y;
+        R dtot = rsub(d, v.y);
         R f = w.F[p];
         w.SF[p] = r2(dtot * f, dtot);
         if (w.SP) w.SP[p] = d * f;
@@ -1110,22 +1125,22 @@ template <typename R> struct Src {
       R s = 0, sa = 0, mx = 0;
       for (int k = 0; k < kl; ++k) {
         const R f = fm[k], a = f * cgs;
-        s = s + f;
-        sa = sa + a;
+        s = radd(s, f);
+        sa = radd(sa, a);
         mx = (k == 0) ? a : dmax(mx, a);
       }
-      R nex = dmax(R(0.0), s * T.DELTH - et) / et;
+      R nex = dmax(R(0.0), rfma(s, T.DELTH, -et)) / et;
       R nex4 = (nex * nex) * (nex * nex);
       T12[m] = R(4.75E-6) * S.FR[m] * nex4;  // T1
       R dfii = (m > 0 && m < nk - 1) ? S.DF[m] * xfac : S.DF[m];
       ADF[m] = nex4 * dfii;
       R s2 = 0;
       if (mx < R(1.0E-34)) s2 = R(kl);
-      else { const R rmx = R(1.) / mx; for (int k = 0; k < kl; ++k) s2 = s2 + (fm[k] * cgs) * rmx; }
+      else { const R rmx = R(1.) / mx; for (int k = 0; k < kl; ++k) s2 = rfma(fm[k] * cgs, rmx, s2); }
       R anar = R(1.0) / (s2 * T.DELTH);
       AB[m] = sa;
       BN[m] = anar * (sa * sig * T.DELTH) * (WN[m] * WN[m] * WN[m]);
-      ps = ps + sa * (P_::ZPI * S.DFIM[m] * sig) / CG[m];
+      ps = radd(ps, sa * (P_::ZPI * S.DFIM[m] * sig) / CG[m]);
       if (sa > amax) { amax = sa; imax = m; }
     }
     __syncwarp();
@@ -1136,7 +1151,7 @@ template <typename R> struct Src {
       R v = (m < nk) ? ADF[m] : R(0);
       for (int o = 1; o < 32; o <<= 1) { R u = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v = v + u; }
       v = v + carry;
-      if (m < nk) T12[m] = R(-1.0) * (dmax(R(0.0), T12[m]) + dmax(R(0.0), R(7.00E-5) * v));
+      if (m < nk) T12[m] = -radd(dmax(R(0.0), T12[m]), dmax(R(0.0), R(7.00E-5) * v));
       carry = __shfl_sync(0xffffffffu, v, 31);
     }
     __syncwarp();
@@ -1157,8 +1172,8 @@ template <typename R> struct Src {
       const int p = k + ld * m;
       const R f = w.F[p];
       R2 v = w.SF[p];
-      v.x = (v.x + T12[m] * f) + AB[m] * f;
-      v.y = (v.y + T12[m]) + AB[m];
+      v.x = rfma(AB[m], f, rfma(T12[m], f, v.x));
+      v.y = radd(radd(v.y, T12[m]), AB[m]);
       w.SF[p] = v;
     });
     __syncwarp();
@@ -1243,7 +1258,7 @@ template <typename R> struct Src {
     // implicit integration with the growth limiter and the minimum-energy floor
     const R delt = T.DELT, fmx = dmax(fmeanws, fmean);
     R* C2 = w.t(2); R* LIM = w.t(3); R* FMIN = w.t(4);  // cos^2 spreading, limiter, floor
-    for (int k = lane; k < kl; k += 32) { R c = dmax(R(0.), dcos(S.TH[k] - UDIR)); C2[k] = c * c; }
+    for (int k = lane; k < kl; k += 32) { R c = dmax(R(0.), dcos(rsub(S.TH[k], UDIR))); C2[k] = c * c; }
     for (int m = lane; m < ml; m += 32) {
       LIM[m] = USTAR * S.DELFL[m] * fmx;
       FMIN[m] = __ldg(&T.FLMINFR[(ju - 1) + 300 * m]);
@@ -1263,10 +1278,10 @@ template <typename R> struct Src {
           R f0 = w.F[p];
           const R2 v = w.SF[p];
           R sl = v.x, fl = v.y;
-          if (T.shallow) { sl = sl + sbo * f0; fl = fl + sbo; }
-          R t1 = fdiv(delt * sl, dmax(R(1.), R(1.) - delt * fl));  // divisor >= 1
+          if (T.shallow) { sl = rfma(sbo, f0, sl); fl = radd(fl, sbo); }
+          R t1 = fdiv(delt * sl, dmax(R(1.), rfma(-delt, fl, R(1.))));  // divisor >= 1
           R t3 = dmin(dabs(t1), lim);
-          R f = f0 + ((t1 >= R(0)) ? t3 : -t3);
+          R f = radd(f0, (t1 >= R(0)) ? t3 : -t3);
           f = dmax(f, fmin * C2[k]);
           w.F[p] = f;
           t = t + f; tw = tw + (w.LL[p] ? f : R(0));

@@ -87,7 +87,7 @@ TileShape tile_shape(const DevTables<float>& T, int max_smem) {
     L.oTab = T.NS * 32;
     L.oU = L.oTab + (T.lay.nreal + 31) / 32 * 32;
     L.oRow = L.oU + u * 32;
-    L.oLL = L.oRow + (st6 ? 4 : 2) * ML * 32;
+    L.oLL = L.oRow + (st6 ? 5 : 2) * ML * 32;
     const int bytes = L.oLL * 4 + ML * (st6 ? (T.KL + 31) / 32 * 128 : L.nw * 32);
     if (bytes <= max_smem) { L.smem = bytes; return L; }
   }

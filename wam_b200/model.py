@@ -354,6 +354,12 @@ class WamModel:
         self._check(0 if w >= 0 else w, "get_halo_width")
         return w
 
+    def implsch_points(self):
+        """Sea points per CTA of IMPLSCH: 32 on tiles, fewer with a warp per point."""
+        n = self.L.wamgpu_get_implsch_points(self.h)
+        self._check(0 if n >= 0 else n, "get_implsch_points")
+        return n
+
     # ---- derivatives (ST4) ---------------------------------------------------
     def implsch_tl_dev(self, fl3, dfl3, tauw, dtauw, u10, du10, udir, roairn, wstar,
                        fl3_out, dfl3_out, tauw_out, dtauw_out, ld=None, stream=None):
