@@ -176,15 +176,19 @@ template <typename R> bool tile_geometry(const TableSet<R>& t) {
 }
 
 // Sea points per IMPLSCH CTA: 32 where the context runs on tiles, else those
-// of the warp-per-point kernel.  Tiles from the first point that the warps no
-// longer hold at once: up to there that kernel takes one wave, and a point of
-// its own per warp is done sooner than a tile (135 points, ST4, KL=24: 151 us
-// against 182; 1485 points, ST6, KL=36: 84 against 121), beyond it takes two and
-// more (1800 points: 302 against 182, 149 against 120).  Both forms give the same
-// bits (implsch.cuh), so a grid's bands, which may fall on the other side,
-// reproduce it.
+// of the warp-per-point kernel.  Both hold a number of points at once and take
+// one wave after the other.  A wave of warps is done sooner than one of tiles (KL=24,
+// 1775 points, one wave each: ST4 159 us against 194, ST6 68 against 81; KL=36: 224
+// against 248, 83 against 134), two waves of warps later (1799 points, KL=24: 293
+// against 194, 116 against 82; KL=36: 397 against 249, 151 against 137).  So a wave of
+// tiles counts 5/4 of one of warps, 7/4 in ST6 with directions beyond 32, where it
+// matters once more between 148 tiles and three waves of warps (4799 points, KL=36,
+// ST6: 236 against 261; KL=24: 189 against 156).  Both forms give the same bits
+// (implsch.cuh), so a grid's bands, which may fall on the other side, reproduce it.
 template <typename R> int cta_points(const wamgpu_ctx* ctx, const DevTables<R>& d) {
-  return d.tile.smem && ctx->nsea > ctx->wave ? 32 : ctx->P;
+  if (!d.tile.smem) return ctx->P;
+  const int warps = (ctx->nsea + ctx->wave - 1) / ctx->wave, tiles = (ctx->nsea + 32 * ctx->nsm - 1) / (32 * ctx->nsm);
+  return tiles * (d.iphys == 2 && d.KL > 32 ? 7 : 5) < warps * 4 ? 32 : ctx->P;
 }
 
 template <typename R> int build_tables(wamgpu_ctx* ctx, Impl<R>& I) {
@@ -432,9 +436,11 @@ template <typename R> int build_tables(wamgpu_ctx* ctx, Impl<R>& I) {
     int ctas = std::min(32 / P, (int)(smpersm / (need + 1024)));
     if (P * ctas > best_warps) { best_warps = P * ctas; ctx->P = P; }
   }
-  ctx->wave = best_warps * ctx->nsm;
   if (ctx->P) CK(implsch_set_max_smem<R>(ctx->P, implsch_smem_bytes(d, ctx->P)), "smem attribute");
   if (!ctx->P) return fail(ctx, WAMGPU_E_ARG, "spectrum too large for the shared-memory workspace");
+  int ctas = 0;
+  CK(implsch_ctas_per_sm<R>(ctx->P, implsch_smem_bytes(d, ctx->P), &ctas), "occupancy");
+  ctx->wave = std::max(1, ctas) * ctx->P * ctx->nsm;
   if constexpr (sizeof(R) == 4) {
     // 1 KB is left to the batched kernel's static part
     if (tile_geometry(t)) d.tile = tile_shape(d, maxsm - 1024);

@@ -191,6 +191,20 @@ template <typename R> cudaError_t implsch_set_max_smem(int P, size_t bytes) {
   return e;
 }
 
+// CTAs of P sea points that an SM holds at once, registers included.
+template <typename R> cudaError_t implsch_ctas_per_sm(int P, size_t bytes, int* ctas) {
+  auto ask = [&](auto kernel) { return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, kernel, 32 * P, bytes); };
+  if (sizeof(R) == 4) {
+    if (P == 4) return ask(implsch_kernel<R, 4>);
+    if (P == 6) return ask(implsch_kernel<R, 6>);
+    if (P == 8) return ask(implsch_kernel<R, 8>);
+  } else {
+    if (P == 2) return ask(implsch_kernel<R, 2>);
+    if (P == 4) return ask(implsch_kernel<R, 4>);
+  }
+  return cudaErrorInvalidValue;
+}
+
 template <typename R> cudaError_t launch_implsch(const DevTables<R>& T, const ImplArgs<R>& a, int P, cudaStream_t s) {
   if (a.nsea == 0) return cudaSuccess;
   if constexpr (sizeof(R) == 4)
@@ -236,6 +250,8 @@ template cudaError_t launch_implsch<float>(const DevTables<float>&, const ImplAr
 template cudaError_t launch_implsch<double>(const DevTables<double>&, const ImplArgs<double>&, int, cudaStream_t);
 template size_t implsch_smem_bytes<float>(const DevTables<float>&, int);
 template size_t implsch_smem_bytes<double>(const DevTables<double>&, int);
+template cudaError_t implsch_ctas_per_sm<float>(int, size_t, int*);
+template cudaError_t implsch_ctas_per_sm<double>(int, size_t, int*);
 template cudaError_t implsch_set_max_smem<float>(int, size_t);
 template cudaError_t implsch_set_max_smem<double>(int, size_t);
 

@@ -59,6 +59,7 @@ cudaError_t launch_implsch_tile_batch(const DevTables<float>& T, const ImplArgs<
                                       int nblocks, cudaStream_t s);
 template <typename R> size_t implsch_smem_bytes(const DevTables<R>& T, int points_per_cta);
 template <typename R> cudaError_t implsch_set_max_smem(int points_per_cta, size_t bytes);
+template <typename R> cudaError_t implsch_ctas_per_sm(int points_per_cta, size_t bytes, int* ctas);
 
 // PROPAGS over the frequency planes m0 .. m0+mcount-1 (mcount < 0: to ML).
 template <typename R>
