@@ -76,10 +76,18 @@ template <typename R> struct PropMember {
   int ld, nbi;
   int pair;  // two frequencies per CTA (propags_pairs)
 };
+bool propags_shallow(int variant);
 // Whether a sub-step takes two frequencies per thread: 32-bit offsets in a plane,
-// and without currents at most eight segments of directions.
+// and without currents at most eight segments of directions.  In double precision
+// only where the halved work outweighs the registers of two frequencies (60k
+// points, pairs against one frequency, us; 36x30 shallow: COUNTER 1 496 against 386,
+// above 551 against 794, with currents 760 against 1196 and 3685 against 2905; 24x25
+// deep: 133 against 179, COUNTER 2 at 12k points 93 against 87, with currents 304
+// against 555 and 1368 against 1354).
 template <typename R> bool propags_pairs(const PropArgs<R>& A, int ld) {
-  return (A.seg[0] > 0 || !propags_planes_independent(A.variant)) && (size_t)ld * A.KL < (size_t(1) << 31);
+  const bool cur = !propags_planes_independent(A.variant);
+  if (sizeof(R) == 8 && (cur ? A.counter > 1 : propags_shallow(A.variant) != (A.counter > 1))) return false;
+  return (A.seg[0] > 0 || cur) && (size_t)ld * A.KL < (size_t(1) << 31);
 }
 // All members of one coefficient family (variant, reduced grid, depth
 // refraction taken from `family`) in one launch of bs-point CTAs (128 or 256);

@@ -646,15 +646,25 @@ cudaError_t dispatch(const PropArgs<R>& A, Args&&... args) {
   return cudaErrorInvalidValue;
 }
 
-// A launch of no more CTAs than this lasts as long as one thread's walk along the
-// directions, which is shorter with one frequency unless there are currents (135
-// points, 36x30, shallow with depth refraction, the call with its copy: 18.6 us
-// against 22.6; with currents 35.0 against 28.8).
-constexpr unsigned PAIR_MIN_CTAS = 32;
+// CTAs of pairs from which on two frequencies per thread are taken.  As long as the
+// CTAs are all resident, a launch lasts as long as one thread's walk along the
+// directions, which is shorter with one frequency (sub-step, pairs against one
+// frequency, us; 36x30 shallow with depth refraction: 720 points, 90 CTAs, 14.5
+// against 12.5; 2000 points, 240 CTAs, 14.7 against 14.6; 3000 points, 360 CTAs, 16.6
+// against 17.5; 24x25 deep: 208 CTAs 11.4 against 10.5, 312 CTAs 12.5 both).  Not so
+// where the walk itself gets shorter: COUNTER above 1 (15 CTAs, shallow 15.5 against
+// 24.8, deep 11.9 against 16.8) and currents (15 CTAs, shallow 18.7 against 24.8;
+// deep 13 CTAs 18.6 against 16.6, 39 CTAs 19.6 against 20.7).  In double precision
+// the line is the same (3000 points, 360 CTAs, COUNTER 2 49 against 54, currents 64
+// against 68; 720 points 43 against 39 and 35 against 33).
+template <typename R, int V> unsigned pairs_from(int counter) {
+  if (sizeof(R) == 8 || (!var_current(V) && counter == 1)) return 257;
+  return var_current(V) && !var_shallow(V) ? 33 : 0;
+}
 template <typename R, int V, bool RED, bool RD> struct PropLaunch {
   static cudaError_t run(const PropArgs<R>& A, const R* f1, int ld1, R* f3, int ld3, int m0, int mcount, cudaStream_t s) {
     const unsigned n = (unsigned)((A.i1 - A.i0 + 127) / 128) * ((mcount + 1) / 2);
-    if (propags_pairs(A, std::max(ld1, ld3)) && (var_current(V) || n > PAIR_MIN_CTAS)) {
+    if (propags_pairs(A, std::max(ld1, ld3)) && n >= pairs_from<R, V>(A.counter)) {
       if constexpr (var_current(V)) {
         // the current's refraction is not switched off by REFRD: one instance
         if (A.counter == 1) propags_pair_cur_kernel<R, V, RED, false, false><<<n, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
@@ -718,6 +728,8 @@ bool propags_planes_independent(int variant) {
   return variant != V_CART_DEEP_CUR && variant != V_CART_SHALLOW_CUR && variant != V_SPHER_DEEP_CURR &&
          variant != V_SPHER_SHALLOW_CURR;
 }
+
+bool propags_shallow(int variant) { return var_shallow(variant); }
 
 template <typename R>
 cudaError_t launch_cfl_extrema(const PropArgs<R>& A, long long* ext, int nsm, cudaStream_t s) {
