@@ -55,7 +55,7 @@ struct wamgpu_ctx {
   cudaStream_t stream = nullptr;
   cudaStream_t copy_stream = nullptr;  // host->device copies overlapped with the kernels of a host-buffer step
   cudaStream_t down_stream = nullptr;  // device->host copies of a host-buffer step
-  cudaStream_t src_stream[4] = {};     // IMPLSCH of the chunks of a host-buffer step (made at its first call)
+  cudaStream_t src_stream[4] = {};     // IMPLSCH of the chunks of a host-buffer step
   std::vector<cudaEvent_t> xfer_ev;     // ordering events between the two streams
   int nsm = 148;
   int P = 8;  // sea points per IMPLSCH CTA of the warp-per-point kernel
@@ -1372,11 +1372,6 @@ int implsch_host_t(wamgpu_ctx* ctx, Impl<R>& I, float* fl3, const float* u10, co
   return wamgpu_sync(ctx);
 }
 
-// Chunks per host<->device copy piece of wamgpu_step_host.  One: pieces of
-// 2 and 4 chunks (longer copy rows) made the regional step 1-4 % slower, the
-// later first download costing more than the rows gained.
-constexpr int kChunksPerCopy = 1;
-
 // Host-buffer form of one WAMODEL pass, with the copies overlapped (see the
 // chunk pipeline below).  Results are identical to the unsplit sequence:
 // every kernel sees the same inputs and writes the same elements.
@@ -1415,11 +1410,11 @@ int step_host_t(wamgpu_ctx* ctx, Impl<R>& I, float* fl3, int nprop, const float*
   // precedes sub-step j+1 of chunk q-1, which overwrites its input; and
   // IMPLSCH of chunk q follows the last sub-step of chunks q-1..q+1.
   const int width = std::max(ctx->halo, 1);
-  // At most 64 chunks, and none below 1184 points (37 tiles of IMPLSCH, a
-  // quarter of the SMs for each of the four in flight) beyond the fourth:
-  // below that the launches bound the step (30k points: 64 chunks 8.2 ms, 32
-  // and 16 chunks 4.7 ms; 756k points: 64 chunks 82 ms, 32 chunks 90 ms).
-  const int nq = n > 0 ? std::min({64, std::max(1, n / width), std::max(4, n / 1184)}) : 1;
+  // At most 64 chunks, and beyond the fourth none that has fewer tiles of IMPLSCH
+  // than a quarter of the SMs, four chunks being in flight: below that the
+  // launches bound the step (30k points: 64 chunks 8.2 ms, 32 and 16 chunks 4.7
+  // ms; 756k points: 64 chunks 82 ms, 32 chunks 90 ms).
+  const int nq = n > 0 ? std::min({64, std::max(1, n / width), std::max(4, n / (8 * ctx->nsm))}) : 1;
   std::vector<int> lo(nq + 1);
   {
     // The first nsub+2 chunks are small (a quarter of the others, and at least
@@ -1436,10 +1431,9 @@ int step_host_t(wamgpu_ctx* ctx, Impl<R>& I, float* fl3, int nprop, const float*
       for (int q = 0; q <= nq; ++q) lo[q] = (int)((long long)n * q / nq);
     }
   }
-  // copies move pieces of kChunksPerCopy chunks
-  const int cpc = kChunksPerCopy, npc = (nq + cpc - 1) / cpc;
-  auto piece_lo = [&](int p) { return lo[std::min(nq, p * cpc)]; };
-  const int nev = 2 * npc + nq;  // uploads, downloads, last sub-steps
+  // a copy moves one chunk (pieces of 2 and 4 chunks, whose copy rows are longer,
+  // made the regional step 1-4 % slower: the first download starts later)
+  const int nev = 3 * nq;  // uploads, IMPLSCH, last sub-steps
   if ((int)ctx->xfer_ev.size() < nev)
     for (int i = (int)ctx->xfer_ev.size(); i < nev; ++i) {
       cudaEvent_t e;
@@ -1447,20 +1441,18 @@ int step_host_t(wamgpu_ctx* ctx, Impl<R>& I, float* fl3, int nprop, const float*
       ctx->xfer_ev.push_back(e);
     }
   cudaStream_t d = ctx->down_stream;
-  for (cudaStream_t& x : ctx->src_stream)
-    if (!x) CK(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking), "stream");
-  // the spectrum piece by piece (the per-point fields went up on s above)
-  for (int p = 0; p < npc; ++p) {
-    const int a0 = piece_lo(p);
-    const size_t w = (size_t)(piece_lo(p + 1) - a0) * 4;
+  // the spectrum chunk by chunk (the per-point fields went up on s above)
+  for (int q = 0; q < nq; ++q) {
+    const int a0 = lo[q];
+    const size_t w = (size_t)(lo[q + 1] - a0) * 4;
     if (w) CK(cudaMemcpy2DAsync(f3 + a0, (size_t)n * 4, fl3 + a0, (size_t)n * 4, w, (size_t)KL * ML,
                                 cudaMemcpyHostToDevice, c), "H2D");
-    CK(cudaEventRecord(ctx->xfer_ev[p], c), "event");
+    CK(cudaEventRecord(ctx->xfer_ev[q], c), "event");
   }
   R* buf[2] = {f3, sc};
   const R* fin = buf[nsub % 2];  // the buffer the last sub-step writes
   auto ready = [&](int q) -> int {  // chunk q and its neighbours are on the device
-    CK(cudaStreamWaitEvent(s, ctx->xfer_ev[std::min(q + 1, nq - 1) / cpc], 0), "wait");
+    CK(cudaStreamWaitEvent(s, ctx->xfer_ev[std::min(q + 1, nq - 1)], 0), "wait");
     return WAMGPU_OK;
   };
   const int last = (nq - 1) + nsub;
@@ -1481,8 +1473,8 @@ int step_host_t(wamgpu_ctx* ctx, Impl<R>& I, float* fl3, int nprop, const float*
     // tiles, far fewer than the SMs, and no later sub-step reads or writes the
     // chunk (those of key t + 1 and on start at chunk q + 2)
     cudaStream_t si = ctx->src_stream[q & 3];
-    CK(cudaEventRecord(ctx->xfer_ev[2 * npc + q], s), "event");
-    CK(cudaStreamWaitEvent(si, ctx->xfer_ev[2 * npc + q], 0), "wait");
+    CK(cudaEventRecord(ctx->xfer_ev[2 * nq + q], s), "event");
+    CK(cudaStreamWaitEvent(si, ctx->xfer_ev[2 * nq + q], 0), "wait");
     if (p1 > p0) {
       ImplArgs<R> a;
       a.nsea = p1 - p0; a.ld = n;
@@ -1498,16 +1490,14 @@ int step_host_t(wamgpu_ctx* ctx, Impl<R>& I, float* fl3, int nprop, const float*
       a.wncg = ctx->wncg_valid ? I.wncg.template as<R>() + (size_t)p0 * 2 * ctx->cfg.ml : nullptr;
       { TimedLaunch tl(ctx, 1, si); CK(launch_implsch<R>(I.dt, a, cta_points(ctx, I.dt), si), "implsch launch"); }
     }
-    if (q % cpc == cpc - 1 || q == nq - 1) {  // the last chunk of a piece: the piece goes down
-      const int pc = q / cpc, a0 = piece_lo(pc);
-      CK(cudaEventRecord(ctx->xfer_ev[npc + pc], si), "event");
-      CK(cudaStreamWaitEvent(d, ctx->xfer_ev[npc + pc], 0), "wait");
-      const size_t w = (size_t)(piece_lo(pc + 1) - a0) * 4;
-      if (w) CK(cudaMemcpy2DAsync(fl3 + a0, (size_t)n * 4, f3 + a0, (size_t)n * 4, w, (size_t)KL * ML,
-                                  cudaMemcpyDeviceToHost, d), "D2H");
-    }
+    // the chunk goes down after its own IMPLSCH
+    CK(cudaEventRecord(ctx->xfer_ev[nq + q], si), "event");
+    CK(cudaStreamWaitEvent(d, ctx->xfer_ev[nq + q], 0), "wait");
+    const size_t w = (size_t)(p1 - p0) * 4;
+    if (w) CK(cudaMemcpy2DAsync(fl3 + p0, (size_t)n * 4, f3 + p0, (size_t)n * 4, w, (size_t)KL * ML,
+                                cudaMemcpyDeviceToHost, d), "D2H");
   }
-  // TAUW, USTAR, Z0 after the last piece (d follows the last IMPLSCH)
+  // TAUW, USTAR, Z0 after the last chunk (d follows every IMPLSCH)
   CK(cudaMemcpyAsync(tauw, I.tauw.template as<R>(), (size_t)n * 4, cudaMemcpyDeviceToHost, d), "D2H");
   CK(cudaMemcpyAsync(ustar, I.ustar.template as<R>(), (size_t)n * 4, cudaMemcpyDeviceToHost, d), "D2H");
   CK(cudaMemcpyAsync(z0, I.z0.template as<R>(), (size_t)n * 4, cudaMemcpyDeviceToHost, d), "D2H");
@@ -1970,6 +1960,8 @@ int wamgpu_create(const wamgpu_config* cfg, wamgpu_ctx** out) {
   if ((e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking)) != cudaSuccess) return bail(cuda_fail(ctx, e, "stream"));
   if ((e = cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking)) != cudaSuccess) return bail(cuda_fail(ctx, e, "stream"));
   if ((e = cudaStreamCreateWithFlags(&ctx->down_stream, cudaStreamNonBlocking)) != cudaSuccess) return bail(cuda_fail(ctx, e, "stream"));
+  for (cudaStream_t& x : ctx->src_stream)
+    if ((e = cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking)) != cudaSuccess) return bail(cuda_fail(ctx, e, "stream"));
   cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, c.device);
   int rc;
   if (c.precision == 8) { auto* I = new Impl<double>(); ctx->impl.reset(I); rc = build_tables<double>(ctx, *I); }
