@@ -290,10 +290,10 @@ template <typename R> struct CurLine {
 // planes m-1 and m+2, which other CTAs own, come from L2 on any grid.  A call on
 // 47k points, 36x30, COUNTER = 1, with its copy of the spectrum: 578 us by the
 // one-frequency kernel, 377 us.
-template <typename R, int VAR, bool RED, bool REFRD, bool CNT>
+template <typename R, int VAR, bool RED, bool CNT>
 __device__ __forceinline__ void propags_pair_cur(const PropArgs<R>& A, const R* __restrict__ f1, int ld1,
                                                  R* __restrict__ f3, int ld3, int i, int m, bool two) {
-  using S = Site<R, VAR, RED, REFRD>;
+  using S = Site<R, VAR, RED, false>;  // the refraction by currents knows no switch
   static_assert(S::CUR, "for the variants with currents");
   constexpr bool SH = S::SH, SPH = S::SPH;
   const int KL = A.KL, mb = min(m + 1, A.ML - 1), mlo = max(m - 1, 0), mhi = two ? min(m + 2, A.ML - 1) : mb;
@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(128) propags_pair_kernel(const __grid_constant
   propags_pair<R, VAR, RED, REFRD, CNT>(A, f1, ld1, f3, ld3, i, m0 + q, q + 1 < mcount);
 }
 
-template <typename R, int VAR, bool RED, bool REFRD, bool CNT>
+template <typename R, int VAR, bool RED, bool CNT>
 __global__ void __launch_bounds__(128) propags_pair_cur_kernel(const __grid_constant__ PropArgs<R> A,
                                                                const R* __restrict__ f1, int ld1, R* __restrict__ f3,
                                                                int ld3, int m0, int mcount) {
@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(128) propags_pair_cur_kernel(const __grid_cons
   const int ib = A.i0 + x * blockDim.x, i = ib + threadIdx.x;
   prefetch_rows(f1, ld1, A.KL, ib, min((int)blockDim.x, A.i1 - ib), m0 + q, q + 1 < mcount);
   if (i >= A.i1) return;
-  propags_pair_cur<R, VAR, RED, REFRD, CNT>(A, f1, ld1, f3, ld3, i, m0 + q, q + 1 < mcount);
+  propags_pair_cur<R, VAR, RED, CNT>(A, f1, ld1, f3, ld3, i, m0 + q, q + 1 < mcount);
 }
 
 // Batched form: every member of an ensemble (one coefficient family) in one
@@ -523,8 +523,8 @@ __global__ void __launch_bounds__(BS) propags_batch_kernel(const PropMember<R>* 
     prefetch_rows(sm.src, sm.ld, sm.A.KL, ib, min(BS, sm.A.i1 - ib), m, two);
     if (i >= sm.A.i1) return;
     if constexpr (Site<R, VAR, RED, REFRD>::CUR) {
-      if (sm.A.counter == 1) propags_pair_cur<R, VAR, RED, REFRD, false>(sm.A, sm.src, sm.ld, sm.dst, sm.ld, i, m, two);
-      else propags_pair_cur<R, VAR, RED, REFRD, true>(sm.A, sm.src, sm.ld, sm.dst, sm.ld, i, m, two);
+      if (sm.A.counter == 1) propags_pair_cur<R, VAR, RED, false>(sm.A, sm.src, sm.ld, sm.dst, sm.ld, i, m, two);
+      else propags_pair_cur<R, VAR, RED, true>(sm.A, sm.src, sm.ld, sm.dst, sm.ld, i, m, two);
     } else {
       if (sm.A.counter == 1) propags_pair<R, VAR, RED, REFRD, false>(sm.A, sm.src, sm.ld, sm.dst, sm.ld, i, m, two);
       else propags_pair<R, VAR, RED, REFRD, true>(sm.A, sm.src, sm.ld, sm.dst, sm.ld, i, m, two);
@@ -666,9 +666,8 @@ template <typename R, int V, bool RED, bool RD> struct PropLaunch {
     const unsigned n = (unsigned)((A.i1 - A.i0 + 127) / 128) * ((mcount + 1) / 2);
     if (propags_pairs(A, std::max(ld1, ld3)) && n >= pairs_from<R, V>(A.counter)) {
       if constexpr (var_current(V)) {
-        // the current's refraction is not switched off by REFRD: one instance
-        if (A.counter == 1) propags_pair_cur_kernel<R, V, RED, false, false><<<n, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
-        else propags_pair_cur_kernel<R, V, RED, false, true><<<n, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
+        if (A.counter == 1) propags_pair_cur_kernel<R, V, RED, false><<<n, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
+        else propags_pair_cur_kernel<R, V, RED, true><<<n, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
       } else if (A.counter == 1) propags_pair_kernel<R, V, RED, RD, false><<<n, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
       else propags_pair_kernel<R, V, RED, RD, true><<<n, 128, 0, s>>>(A, f1, ld1, f3, ld3, m0, mcount);
       return cudaGetLastError();

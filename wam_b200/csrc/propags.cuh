@@ -5,11 +5,11 @@
 // per-point metadata (depth-table indices, gradients, metric factors), so a
 // sub-step moves only the spectrum itself: one read and one write per bin.
 //
-// Thread layout: one thread per (sea point, frequency), looping over the
-// directions; the direction neighbours K+-1 needed by the refraction terms are
-// kept in a register window.  Consecutive threads handle consecutive sea
-// points, so every access to FL3(IJ,K,M) is coalesced; the north/south
-// neighbours of a latitude row are re-read from L2.
+// Thread layout: one thread per sea point and one or two frequencies (which, and
+// where: pairs_from in propags.cu, propags_pairs), looping over the directions; the
+// direction neighbours K+-1 needed by the refraction terms are kept in registers.
+// Consecutive threads handle consecutive sea points, so every access to FL3(IJ,K,M)
+// is coalesced; the north/south neighbours of a latitude row are re-read from L2.
 //
 // Direction sines and cosines travel in the metadata block itself (a
 // __grid_constant__ kernel parameter), so grids with different KL can live
