@@ -55,7 +55,7 @@ struct wamgpu_ctx {
   cudaStream_t stream = nullptr;
   cudaStream_t copy_stream = nullptr;  // host->device copies overlapped with the kernels of a host-buffer step
   cudaStream_t down_stream = nullptr;  // device->host copies of a host-buffer step
-  cudaStream_t src_stream[4] = {};     // IMPLSCH of the chunks of a host-buffer step
+  cudaStream_t src_stream[4] = {};     // IMPLSCH of the chunks of a host-buffer step (made at its first call)
   std::vector<cudaEvent_t> xfer_ev;     // ordering events between the two streams
   int nsm = 148;
   int P = 8;  // sea points per IMPLSCH CTA of the warp-per-point kernel
@@ -1441,6 +1441,9 @@ int step_host_t(wamgpu_ctx* ctx, Impl<R>& I, float* fl3, int nprop, const float*
       ctx->xfer_ev.push_back(e);
     }
   cudaStream_t d = ctx->down_stream;
+  // made here: four streams take 0.8 ms, which every other context would pay too
+  for (cudaStream_t& x : ctx->src_stream)
+    if (!x) CK(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking), "stream");
   // the spectrum chunk by chunk (the per-point fields went up on s above)
   for (int q = 0; q < nq; ++q) {
     const int a0 = lo[q];
@@ -1960,8 +1963,6 @@ int wamgpu_create(const wamgpu_config* cfg, wamgpu_ctx** out) {
   if ((e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking)) != cudaSuccess) return bail(cuda_fail(ctx, e, "stream"));
   if ((e = cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking)) != cudaSuccess) return bail(cuda_fail(ctx, e, "stream"));
   if ((e = cudaStreamCreateWithFlags(&ctx->down_stream, cudaStreamNonBlocking)) != cudaSuccess) return bail(cuda_fail(ctx, e, "stream"));
-  for (cudaStream_t& x : ctx->src_stream)
-    if ((e = cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking)) != cudaSuccess) return bail(cuda_fail(ctx, e, "stream"));
   cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, c.device);
   int rc;
   if (c.precision == 8) { auto* I = new Impl<double>(); ctx->impl.reset(I); rc = build_tables<double>(ctx, *I); }
