@@ -40,3 +40,28 @@ def test_whole_launch_equals_small_ranges(kl, ml, shallow, refr_d, currents, ide
     m.sync()
     assert torch.equal(a, b), int((a != b).sum())
     m.close()
+
+
+@pytest.mark.parametrize("idelpro", [3600, 14400])
+@pytest.mark.parametrize("spherical,shallow,reduced,refr_d", [(0, 0, 0, 0), (0, 1, 0, 1), (1, 0, 0, 0), (1, 0, 1, 0), (1, 1, 0, 0),
+                                                              (1, 1, 1, 1)])
+def test_quotients_by_counter_match_the_oracle(oracle_mod, spherical, shallow, reduced, refr_d, idelpro):
+    """Without currents every coefficient is divided by COUNTER as a scaled
+    quotient of its own: bit for bit the oracle's division."""
+    from test_gpu_propags_variants import _case
+    from wam_b200 import WamModel
+    cfg, g, depth, _, _, f = _case(oracle_mod, spherical, shallow, 0, reduced, refr_d, idelpro=idelpro)
+    o = oracle_mod.Oracle(cfg)
+    o.set_grid(g)
+    o.set_fields(depth)
+    rc, _, cnt = o.prepare_propagation()
+    assert rc == 0 and cnt > 1
+    m = WamModel(cfg)
+    m.set_grid(g)
+    m.set_depth(depth)
+    m.prepare_propagation()
+    ref = o.propags(f.astype(float)).astype(np.float32)
+    got = f.copy(order="F")
+    m.propags(got)
+    assert np.array_equal(got, ref), float(np.abs(got - ref).max())
+    m.close()
