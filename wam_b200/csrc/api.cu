@@ -1792,7 +1792,7 @@ struct Branches {
 // One pass of all members.  With branches (capture) every source-table class but
 // the first runs IMPLSCH on a branch of its own: a class is a few waves of tiles,
 // one per SM, whose last wave leaves most SMs idle, and the next class fills
-// them.  Eight members of 1k-47k points in four classes: 5.08 -> 4.94 ms a pass.
+// them.  Eight members of 1k-47k points in four classes: 5.51 -> 5.38 ms a pass.
 template <typename R> int batch_launch(wamgpu_batch* b, cudaStream_t s, Branches* br = nullptr) {
   for (auto& step : b->sub)
     for (auto& L : step) {
